@@ -436,7 +436,8 @@ vmap_status build_map(const vmap_config& cfg, unsigned char* base, cudaStream_t 
     m->dm.mu = cfg.truncation;
     m->dm.wmax = (float)cfg.max_weight;
     m->epoch = 0xFFFFFFFEu;  // the first render re-initialises the tiles
-    vmap_status st = vmap_reset(m, stream);
+    vmap_status st = VMAP_OK;  // the memory may hold anything: clear the whole pool
+    if ((e = launch_reset(m->dm, true, m->launcher, stream)) != cudaSuccess) st = cuda_fail(e, "create reset");
     if (st == VMAP_OK && !base && (e = cudaStreamSynchronize(stream)) != cudaSuccess) st = cuda_fail(e, "create sync");
     if (st != VMAP_OK) {
         free_all(m);
@@ -520,7 +521,7 @@ vmap_status vmap_get_config(const vmap_map* m, vmap_config* out)
 vmap_status vmap_reset(vmap_map* m, void* stream)
 {
     if (!m) return VMAP_ERR_INVALID_ARG;
-    VMAP_CK(launch_reset(m->dm, m->poolBytes, m->launcher, as_stream(stream)));
+    VMAP_CK(launch_reset(m->dm, false, m->launcher, as_stream(stream)));
     return VMAP_OK;
 }
 

@@ -111,7 +111,7 @@ template <class V>
 cudaError_t launch_visibility(const V& views, const Launcher& l, cudaStream_t s);
 template <class V>
 cudaError_t launch_fuse(const V& views, int fmt, const Launcher& l, cudaStream_t s);
-cudaError_t launch_reset(const DevMap& m, size_t poolBytes, const Launcher& l, cudaStream_t s);
+cudaError_t launch_reset(const DevMap& m, bool whole, const Launcher& l, cudaStream_t s);
 
 // raycast.cu
 template <class V>
