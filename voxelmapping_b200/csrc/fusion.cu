@@ -111,21 +111,31 @@ __global__ void __launch_bounds__(256, 6) fuse_kernel(V views)
 }
 
 // ------------------------------------------------------------------- reset
-// MapStruct::reset (map_struct.cu:29-42): empty hash slots, zeroed voxels. A
+// MapStruct::reset (map_struct.cu:29-42): empty hash slots and grid, zeroed voxels. A
 // pool block is written only after it has been handed out, so only the
 // allocated blocks hold anything to clear (all of them after a snapshot load
 // that stopped half-way). Bound by the bytes it writes: emptying a 2^20-block
 // FP32 + colour map (5.9 GB pool, 60 MB hash table) that holds 8k blocks,
 // fusing a frame and rendering it takes 166 us; 958 us with the whole pool
 // cleared each time.
-__global__ void __launch_bounds__(256) reset_kernel(DevMap m, bool pool)
+__global__ void __launch_bounds__(256) reset_kernel(DevMap m, bool whole)
 {
     const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x, nt = (size_t)gridDim.x * blockDim.x;
     const size_t slots = (size_t)m.nBucket * kSlots;
     for (size_t i = t; i < slots; i += nt) m.slots[i] = make_ulonglong2(kEmptyKey, ~0ull);
-    if (!pool) return;
+    const bool unknown = whole || m.ctr[C_UNKNOWN];
+    if (unknown) {
+        const size_t cells = grid_cells(m.capacity);
+        for (size_t i = t; i < cells; i += nt) m.grid[i] = 0ull;
+        for (size_t i = t; i < cells / 64; i += nt) m.occ[i] = 0ull;
+        for (size_t i = t; i < cells / 4096; i += nt) m.occ2[i] = 0ull;
+    } else {
+        const int n = allocated_blocks(m);
+        for (size_t i = t; i < (size_t)n; i += nt) grid_clear(m, m.blockKeys[i]);
+    }
+    if (whole) return;  // the host clears the pool
     // block bytes are a multiple of 16 in every format, and the pool is 256-byte aligned
-    const size_t blocks = m.ctr[C_UNKNOWN] ? (size_t)m.capacity : (size_t)allocated_blocks(m);
+    const size_t blocks = unknown ? (size_t)m.capacity : (size_t)allocated_blocks(m);
     const size_t words = blocks * (size_t)m.blockBytes / sizeof(uint4);
     uint4* w = reinterpret_cast<uint4*>(m.pool);
     for (size_t i = t; i < words; i += nt) w[i] = make_uint4(0u, 0u, 0u, 0u);
@@ -168,7 +178,7 @@ template cudaError_t launch_fuse<ManyViews>(const ManyViews&, int, const Launche
 // not tell what to clear.
 cudaError_t launch_reset(const DevMap& m, bool whole, const Launcher& l, cudaStream_t s)
 {
-    reset_kernel<<<l.numSMs * 8, 256, 0, s>>>(m, !whole);
+    reset_kernel<<<l.numSMs * 8, 256, 0, s>>>(m, whole);
     cudaError_t e = cudaGetLastError();
     if (e == cudaSuccess && whole) e = cudaMemsetAsync(m.pool, 0, (size_t)m.capacity * m.blockBytes, s);
     if (e != cudaSuccess) return e;

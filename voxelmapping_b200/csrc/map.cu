@@ -20,6 +20,7 @@ struct vmap_map {
     Launcher launcher;
     int device;
     bool external;            // device buffers live in caller memory (vmap_create_in)
+    unsigned char* arena;     // else in this one allocation
     size_t poolBytes;
     size_t deviceBytes;
     unsigned* hCtr;           // pinned readback of the counters
@@ -90,6 +91,26 @@ bool pose_ok(const double p[16])
 }  // namespace
 
 namespace vmapb {
+// How far the view's ray samples get from the world's origin on any axis, in
+// voxels: every sample lies between a ray's start and end, and the farthest of
+// these points belong to the image corners.
+static double view_reach(const vmap_map* m, const double pose[16])
+{
+    const vmap_config& c = m->cfg;
+    double reach = 0;
+    for (int k = 0; k < 8; ++k) {
+        const double z = k & 4 ? kMaxDepth : kMinDepth;
+        const double x = ((k & 1 ? c.width : -1) - c.cx) / c.fx * z, y = ((k & 2 ? c.height : -1) - c.cy) / c.fy * z;
+        for (int i = 0; i < 3; ++i) {
+            const double* r = pose + 4 * i;
+            const double p = std::fabs(r[0] * x + r[1] * y + r[2] * z + r[3]) / c.voxel_size;
+            if (!std::isfinite(p)) return HUGE_VAL;
+            reach = std::fmax(reach, p);
+        }
+    }
+    return reach;
+}
+
 // The per-step view of a map: storage, camera, pose (FP64 inverse rounded to
 // FP32), no frame inputs and no render outputs yet.
 void make_view(const vmap_map* m, const double pose[16], MapView& v)
@@ -117,7 +138,15 @@ void make_view(const vmap_map* m, const double pose[16], MapView& v)
     v.out.zmin = m->zmin;
     v.out.zmax = m->zmax;
     v.out.vsinv = (float)(1.0 / (double)m->cfg.voxel_size);
+    v.out.vsinvRcp = 1.f / v.out.vsinv;
     v.out.rts = m->cfg.truncation / m->cfg.voxel_size;
+    if (pose) {
+        const double reach = view_reach(m, pose);
+        v.out.wide = !(reach < narrow_limit(m->dm.gridLog2));
+        // a jump rounds a position by half a unit in the last place, 2^-24 of
+        // it; a cube is crossed in some 50 jumps at most
+        v.out.slack = (float)(0.05 + reach * 0x1p-17);
+    }
     v.out.mode = m->cfg.raycast_mode;
 }
 
@@ -213,17 +242,7 @@ void free_all(vmap_map* m)
 {
     timing_free(m);
     pipe_free(m);
-    if (!m->external) {  // buffers carved from caller memory stay with the caller
-        cudaFree(m->dm.slots);
-        cudaFree(m->dm.blockKeys);
-        cudaFree(m->dm.pool);
-        cudaFree(m->dm.ctr);
-        cudaFree(m->dm.visList);
-        cudaFree(m->zmin);
-        cudaFree(m->zmax);
-        cudaFree(m->dNtri);
-        cudaFree(m->dm.nbr);
-    }
+    cudaFree(m->arena);
     cudaFree(m->dDepth);
     cudaFree(m->dRgb);
     cudaFree(m->dVmap);
@@ -356,9 +375,10 @@ vmap_status resolve_config(const vmap_config* cfg_in, vmap_config& cfg)
 
 // Device buffers of a map, in order, each starting on a 256-byte boundary:
 // hash slots, block keys, voxel pool, counters, visible list, z-range tiles
-// (min, max), triangle count.
+// (min, max), triangle count, neighbour links, block grid (bricks,
+// regions, cells).
 struct MapLayout {
-    enum { SLOTS, KEYS, POOL, CTR, VIS, ZMIN, ZMAX, NTRI, NBR, N };
+    enum { SLOTS, KEYS, POOL, CTR, VIS, ZMIN, ZMAX, NTRI, NBR, OCC, OCC2, GRID, N };
     size_t off[N + 1];
 };
 
@@ -370,7 +390,10 @@ MapLayout map_layout(const vmap_config& cfg)
                                      cap * vmap_block_bytes(cfg.voxel_format, cfg.with_color),
                                      C_COUNT * sizeof(unsigned), cap * sizeof(int),
                                      ntiles * sizeof(unsigned long long), ntiles * sizeof(unsigned long long),
-                                     sizeof(unsigned), cap * 7 * sizeof(int)};
+                                     sizeof(unsigned), cap * 7 * sizeof(int),
+                                     grid_cells(cfg.num_blocks) / 64 * sizeof(unsigned long long),
+                                     grid_cells(cfg.num_blocks) / 4096 * sizeof(unsigned long long),
+                                     grid_cells(cfg.num_blocks) * sizeof(unsigned long long)};
     MapLayout l;
     l.off[0] = 0;
     for (int i = 0; i < MapLayout::N; ++i) l.off[i + 1] = (l.off[i] + sz[i] + 255) / 256 * 256;
@@ -379,8 +402,9 @@ MapLayout map_layout(const vmap_config& cfg)
 
 // Builds a map for a resolved configuration. With `base` non-NULL its device
 // buffers are carved from the caller's memory (MapLayout) and the reset runs
-// asynchronously on `stream`; otherwise they are cudaMalloc'ed and the reset
-// is synchronous.
+// asynchronously on `stream`; otherwise from one allocation of the map's own (an
+// allocation each made a map's creation up to 3 ms longer), and the reset is
+// synchronous.
 vmap_status build_map(const vmap_config& cfg, unsigned char* base, cudaStream_t stream, vmap_map** out)
 {
     int dev = 0;
@@ -409,19 +433,20 @@ vmap_status build_map(const vmap_config& cfg, unsigned char* base, cudaStream_t 
     const MapLayout l = map_layout(cfg);
     void** ptrs[MapLayout::N] = {(void**)&m->dm.slots, (void**)&m->dm.blockKeys, (void**)&m->dm.pool,
                                  (void**)&m->dm.ctr, (void**)&m->dm.visList, (void**)&m->zmin, (void**)&m->zmax,
-                                 (void**)&m->dNtri, (void**)&m->dm.nbr};
-    for (int i = 0; i < MapLayout::N; ++i) {
-        const size_t bytes = l.off[i + 1] - l.off[i];
-        if (base) {
-            *ptrs[i] = base + l.off[i];
-            m->deviceBytes += bytes;
-        } else if ((e = dalloc(m, (unsigned char**)ptrs[i], bytes)) != cudaSuccess) {
+                                 (void**)&m->dNtri, (void**)&m->dm.nbr, (void**)&m->dm.occ, (void**)&m->dm.occ2,
+                                 (void**)&m->dm.grid};
+    if (base) {
+        m->deviceBytes = l.off[MapLayout::N];
+    } else {
+        if ((e = dalloc(m, &m->arena, l.off[MapLayout::N])) != cudaSuccess) {
             vmap_status st = cuda_fail(e, "cudaMalloc");
             free_all(m);
             delete m;
             return st;
         }
+        base = m->arena;
     }
+    for (int i = 0; i < MapLayout::N; ++i) *ptrs[i] = base + l.off[i];
     if ((e = cudaHostAlloc((void**)&m->hCtr, C_COUNT * sizeof(unsigned), cudaHostAllocDefault)) != cudaSuccess) {
         vmap_status st = cuda_fail(e, "cudaHostAlloc");
         free_all(m);
@@ -431,6 +456,7 @@ vmap_status build_map(const vmap_config& cfg, unsigned char* base, cudaStream_t 
     m->dm.nBucket = cfg.num_buckets;
     m->dm.bucketMagic = bucket_magic((unsigned)cfg.num_buckets);
     m->dm.capacity = cfg.num_blocks;
+    m->dm.gridLog2 = grid_log2(cfg.num_blocks);
     m->dm.blockBytes = (int)blockBytes;
     m->dm.vs = cfg.voxel_size;
     m->dm.mu = cfg.truncation;
@@ -438,7 +464,7 @@ vmap_status build_map(const vmap_config& cfg, unsigned char* base, cudaStream_t 
     m->epoch = 0xFFFFFFFEu;  // the first render re-initialises the tiles
     vmap_status st = VMAP_OK;  // the memory may hold anything: clear the whole pool
     if ((e = launch_reset(m->dm, true, m->launcher, stream)) != cudaSuccess) st = cuda_fail(e, "create reset");
-    if (st == VMAP_OK && !base && (e = cudaStreamSynchronize(stream)) != cudaSuccess) st = cuda_fail(e, "create sync");
+    if (st == VMAP_OK && !m->external && (e = cudaStreamSynchronize(stream)) != cudaSuccess) st = cuda_fail(e, "create sync");
     if (st != VMAP_OK) {
         free_all(m);
         delete m;
@@ -621,7 +647,7 @@ vmap_status vmap_render_scene(vmap_map* m, const double pose[16], float* vmap_de
     // the z-range kernel also rewinds the raycast work queue, so it runs in
     // both raycast modes (with no work in mode 1)
     VMAP_CK(staged(m, VMAP_STAGE_ZRANGE, s, [&] { return launch_zrange(ov, m->launcher, s); }));
-    VMAP_CK(staged(m, VMAP_STAGE_RAYCAST, s, [&] { return launch_raycast(ov, m->cfg.voxel_format, m->launcher, s); }));
+    VMAP_CK(staged(m, VMAP_STAGE_RAYCAST, s, [&] { return launch_raycast(ov, m->cfg.voxel_format, ov.v.out.wide != 0, m->launcher, s); }));
     if (nmap_dev)
         VMAP_CK(staged(m, VMAP_STAGE_NORMALS, s, [&] {
             return launch_normals(ov, stage_tiles(m->cfg.width, m->cfg.height), m->launcher, s);

@@ -1,6 +1,6 @@
 // Ray marcher device code (MapRenderingDelegate, src/ray_tracing.cu:255-401)
 // shared by the ray-marching kernel and the persistent batch step: per-ray
-// state, the sample loop, the per-warp block cache and one warp's tile.
+// state, the sample loop and one warp's tile.
 #pragma once
 
 #include "vmap_launch.h"
@@ -21,22 +21,46 @@ __device__ __forceinline__ float3 fma3(float k, float3 d, float3 r)
     return make_float3(__fmaf_rn(k, d.x, r.x), __fmaf_rn(k, d.y, r.y), __fmaf_rn(k, d.z, r.z));
 }
 
-// Per-lane state of one ray.
+// Per-lane state of one ray. cx, cy, cz: floor codes (March::fl) of a voxel in
+// the region that the last lookup settled: the aligned cube of side cmask + 1
+// voxels, 8 (one block) with its slot in cblk, or 8, 32 or 128 that hold no
+// allocated block (cblk -1). bits: occupancy word of that voxel's brick.
 struct Ray {
-    int mi;            // map index, -1 = lane idle
     int x, y;
     float3 res, dir, inv;
     float dist_s, dist_lim;
     float sdf;
     bool valid;
-    int cbx, cby, cbz, cblk;  // block of the current sample
-    int obx, oby, obz, oblk;  // last other block (trilinear corners)
+    int cx, cy, cz, cmask, cblk;
+    unsigned long long bits;
 };
 
-template <int FMT, bool NC = true>
+// WIDE: some ray of the view may leave the narrow range (narrow_limit, set per
+// view by the host from the image corners). Otherwise a floor is one full-rate add,
+// rounded down, of 1.5 * 2^23: the low 22 bits of the sum are floor(p), and
+// subtracting the constant again gives it as a float, both exact below 2^22.
+// The conversion instructions that do the same run at a quarter of the rate or
+// less, and a trilinear sample needs a dozen of them.
+template <int FMT, bool NC, bool WIDE>
 struct March {
     typedef Fmt<FMT> F;
     typedef typename F::Word Word;
+    static constexpr float kFloorAdd = 12582912.f;  // 1.5 * 2^23
+
+    // floor(p) as an integer code: equal in the low 22 bits, differences exact
+    static __device__ __forceinline__ int fl(float p)
+    {
+        if constexpr (WIDE) return __float2int_rd(p);
+        else return __float_as_int(__fadd_rd(p, kFloorAdd));
+    }
+    // the code as a float
+    static __device__ __forceinline__ float ff(int i)
+    {
+        if constexpr (WIDE) return __int2float_rn(i);
+        else return __fsub_rn(__int_as_float(i), kFloorAdd);
+    }
+    // voxel index in its block
+    static __device__ __forceinline__ int at(int ix, int iy, int iz) { return local_idx(ix, iy, iz); }
 
     // read_sdf (ray_tracing.cu:272-286) on a loaded word
     static __device__ __forceinline__ float value(Word w, bool& valid)
@@ -45,22 +69,28 @@ struct March {
         return valid ? F::tsdf(w) : 1.f;
     }
 
-    static __device__ __forceinline__ float voxel(const DevMap& m, int slot, int vx, int vy, int vz, bool& valid)
+    static __device__ __forceinline__ float voxel(const DevMap& m, int slot, int ix, int iy, int iz, bool& valid)
     {
-        if (slot >= 0) return value(ld_map<NC>(Layout<FMT>::words(m, slot) + local_idx(vx, vy, vz)), valid);
+        if (slot >= 0) return value(ld_map<NC>(Layout<FMT>::words(m, slot) + at(ix, iy, iz)), valid);
         valid = false;
         return 1.f;
     }
 
-    static __device__ __forceinline__ int block_of(const DevMap& m, Ray& r, int bx, int by, int bz)
+    // Grid entry of the block of floor codes (ix, iy, iz), and the slot it
+    // gives (-1: absent). Narrow codes are not the coordinates, but agree with
+    // them in the bits that the cell and the tag use.
+    static __device__ __forceinline__ unsigned long long entry(const DevMap& m, int ix, int iy, int iz)
     {
-        if (bx == r.cbx && by == r.cby && bz == r.cbz) return r.cblk;
-        if (bx == r.obx && by == r.oby && bz == r.obz) return r.oblk;
-        r.obx = bx;
-        r.oby = by;
-        r.obz = bz;
-        r.oblk = hash_find<NC>(m, bx, by, bz);
-        return r.oblk;
+        const int bx = ix >> 3, by = iy >> 3, bz = iz >> 3;
+        return ld_map<NC>(m.grid + ((size_t)grid_brick(m, bx, by, bz) * 64 + grid_bit(bx, by, bz)));
+    }
+    static __device__ __forceinline__ int slot_of(const DevMap& m, unsigned long long e, int ix, int iy, int iz)
+    {
+        const int bx = ix >> 3, by = iy >> 3, bz = iz >> 3;
+        const unsigned hi = (unsigned)(e >> 32), tag = WIDE ? grid_tag(m, bx, by, bz) : grid_tag_bits(m, bx, by, bz);
+        if ((!WIDE || tag) && (hi & ~kGridShared) == tag) return (int)(unsigned)e;
+        constexpr int k = WIDE ? 0 : __builtin_bit_cast(int, kFloorAdd) >> 3;
+        return hi & kGridShared ? hash_find<NC>(m, bx - k, by - k, bz - k) : -1;
     }
 
     // read_sdf_interped (ray_tracing.cu:288-321): corners floor(p + {0,1}^3),
@@ -77,139 +107,123 @@ struct March {
         return __fmaf_rn(bz, r2, __fmul_rn(az, r3));
     }
 
+    // Corners of a trilinear read: fractions and the floor codes of p and p + 1.
     struct Corners {
         float ax, ay, az;
         int x0, y0, z0, x1, y1, z1;
-        __device__ __forceinline__ bool inner() const  // all 8 corners in the block of (x0, y0, z0)
+        // axes on which corner 1 lies in another block than corner 0 (bits
+        // 0-2): the voxels are 1 or 2 apart, so bit 3 tells
+        __device__ __forceinline__ int cross() const
         {
-            return x1 == x0 + 1 && y1 == y0 + 1 && z1 == z0 + 1 && (x0 & 7) != 7 && (y0 & 7) != 7 && (z0 & 7) != 7;
+            return ((x0 ^ x1) >> 3 & 1) | ((y0 ^ y1) >> 2 & 2) | ((z0 ^ z1) >> 1 & 4);
         }
     };
 
-    // The voxel floor(p) of a sample: all the loop head needs (the block
-    // lookup and the first read). The trilinear fractions and far corners are
-    // computed from the same position only on the samples that interpolate,
-    // so they are not live across the warp's block lookup.
-    struct Cell {
-        int x0, y0, z0;
-    };
-
-    static __device__ __forceinline__ Cell cell(float3 p)
-    {
-        Cell c;
-        c.x0 = __float2int_rz(floorf(p.x));
-        c.y0 = __float2int_rz(floorf(p.y));
-        c.z0 = __float2int_rz(floorf(p.z));
-        return c;
-    }
-
-    static __device__ __forceinline__ Corners corners(float3 p)
+    static __device__ __forceinline__ Corners corners(float3 p, int ix, int iy, int iz)
     {
         Corners c;
-        const float flx = floorf(p.x), fly = floorf(p.y), flz = floorf(p.z);
-        c.ax = __fsub_rn(p.x, flx);
-        c.ay = __fsub_rn(p.y, fly);
-        c.az = __fsub_rn(p.z, flz);
-        c.x0 = __float2int_rz(flx);
-        c.y0 = __float2int_rz(fly);
-        c.z0 = __float2int_rz(flz);
-        c.x1 = __float2int_rz(floorf(__fadd_rn(p.x, 1.f)));
-        c.y1 = __float2int_rz(floorf(__fadd_rn(p.y, 1.f)));
-        c.z1 = __float2int_rz(floorf(__fadd_rn(p.z, 1.f)));
+        c.x0 = ix;
+        c.y0 = iy;
+        c.z0 = iz;
+        c.ax = __fsub_rn(p.x, ff(ix));
+        c.ay = __fsub_rn(p.y, ff(iy));
+        c.az = __fsub_rn(p.z, ff(iz));
+        c.x1 = fl(__fadd_rn(p.x, 1.f));
+        c.y1 = fl(__fadd_rn(p.y, 1.f));
+        c.z1 = fl(__fadd_rn(p.z, 1.f));
         return c;
     }
 
-    // 8 corner values from one block with independent loads; returns the
-    // mask of observed corners (bit k = corner k)
-    static __device__ __forceinline__ unsigned load8(const DevMap& m, int slot, const Corners& c, float* s)
+    // Slot of the block that holds the far corners when they leave corner 0's
+    // block `slot` on exactly one axis, `slot` itself when they do not leave
+    // it: read together with the sample, so the corners' own reads need not
+    // wait for it.
+    static __device__ __forceinline__ int far_slot(const DevMap& m, int slot, int cross)
     {
-        const Word* w = Layout<FMT>::words(m, slot) + local_idx(c.x0, c.y0, c.z0);
-        const Word w0 = ld_map<NC>(w), w1 = ld_map<NC>(w + 1), w2 = ld_map<NC>(w + 8), w3 = ld_map<NC>(w + 9);
-        const Word w4 = ld_map<NC>(w + 64), w5 = ld_map<NC>(w + 65), w6 = ld_map<NC>(w + 72), w7 = ld_map<NC>(w + 73);
-        unsigned mask = 0;
-        bool v;
-        s[0] = value(w0, v); mask |= (unsigned)v;
-        s[1] = value(w1, v); mask |= (unsigned)v << 1;
-        s[2] = value(w2, v); mask |= (unsigned)v << 2;
-        s[3] = value(w3, v); mask |= (unsigned)v << 3;
-        s[4] = value(w4, v); mask |= (unsigned)v << 4;
-        s[5] = value(w5, v); mask |= (unsigned)v << 5;
-        s[6] = value(w6, v); mask |= (unsigned)v << 6;
-        s[7] = value(w7, v); mask |= (unsigned)v << 7;
-        return mask;
+        return cross == 1 || cross == 2 || cross == 4 ? ld_map<NC>(m.nbr + (7 * (size_t)slot + cross - 1)) : slot;
     }
 
-    // corners across block boundaries, from the block of corner 0 (slot0)
-    // and its forward neighbour links: floor(p + 1) is floor(p) + 1 or + 2,
-    // so the other corners lie in that block or in a block one step up on
-    // each axis that crosses; the needed links are independent loads
-    static __device__ __forceinline__ bool load8_linked(const DevMap& m, int slot0, const Corners& c, float* s)
+    // Values of the 8 corners of c, all observed or not, from corner 0's block
+    // `slot` (allocated), its far block and, for corners that leave it on
+    // several axes, its forward neighbour links. w0: corner 0's word.
+    //
+    // Where at most one axis leaves the block, corner k's address is corner
+    // 0's plus one byte offset per axis, whether that axis steps inside the
+    // block or into the far one, so every lane of the warp issues the same 7
+    // independent loads, where a branch per block layout took a round trip to
+    // L2 each. floor(p + 1) is floor(p) + 1 or + 2, hence the general in-block
+    // offsets. (All 8 corners read with every sample, to save the round trip
+    // after it, measured 15-25 % slower: at full size instructions bound it.)
+    static __device__ __forceinline__ bool corners8(const DevMap& m, int slot, int far, int cross, const Corners& c, Word w0,
+                                                    float* s)
     {
-        const int mask = (vox2blk(c.x1) != vox2blk(c.x0) ? 1 : 0) | (vox2blk(c.y1) != vox2blk(c.y0) ? 2 : 0) |
-                         (vox2blk(c.z1) != vox2blk(c.z0) ? 4 : 0);
-        const int* L = m.nbr + 7 * (size_t)slot0;
-        bool ok = true;
+        bool ok, v;
+        s[0] = value(w0, ok);
+        if (cross == 0 || cross == 1 || cross == 2 || cross == 4) {
+            const bool gone = far < 0;  // the far corners' block is not allocated
+            const long long hop = gone ? 0ll : (long long)(far - slot) * m.blockBytes;
+            const char* a = reinterpret_cast<const char*>(Layout<FMT>::words(m, slot) + at(c.x0, c.y0, c.z0));
+            const char* ax = a + ((c.x1 & 7) - (c.x0 & 7)) * (int)sizeof(Word) + (cross == 1 ? hop : 0ll);
+            const long long dy = ((c.y1 & 7) - (c.y0 & 7)) * 8 * (int)sizeof(Word) + (cross == 2 ? hop : 0ll);
+            const long long dz = ((c.z1 & 7) - (c.z0 & 7)) * 64 * (int)sizeof(Word) + (cross == 4 ? hop : 0ll);
+            auto ld = [](const char* p) { return ld_map<NC>(reinterpret_cast<const Word*>(p)); };
+            const Word w1 = ld(ax), w2 = ld(a + dy), w3 = ld(ax + dy), w4 = ld(a + dz), w5 = ld(ax + dz);
+            const Word w6 = ld(a + dy + dz), w7 = ld(ax + dy + dz);
+            s[1] = value(w1, v); ok &= v;
+            s[2] = value(w2, v); ok &= v;
+            s[3] = value(w3, v); ok &= v;
+            s[4] = value(w4, v); ok &= v;
+            s[5] = value(w5, v); ok &= v;
+            s[6] = value(w6, v); ok &= v;
+            s[7] = value(w7, v); ok &= v;
+            if (gone) {
 #pragma unroll
-        for (int k = 0; k < 8; ++k) {
-            const int vx = (k & 1) ? c.x1 : c.x0, vy = (k & 2) ? c.y1 : c.y0, vz = (k & 4) ? c.z1 : c.z0;
-            const int o = k & mask;  // corner k's block, as an offset from corner 0's
-            bool v;
-            s[k] = voxel(m, o ? ld_map<NC>(L + o - 1) : slot0, vx, vy, vz, v);
-            ok &= v;
+                for (int k = 1; k < 8; ++k)
+                    if (k & cross) s[k] = 1.f;
+                ok = false;
+            }
+        } else {  // several axes: independent links, then independent corners
+            const int* L = m.nbr + 7 * (size_t)slot;
+#pragma unroll
+            for (int k = 1; k < 8; ++k) {
+                const int vx = (k & 1) ? c.x1 : c.x0, vy = (k & 2) ? c.y1 : c.y0, vz = (k & 4) ? c.z1 : c.z0;
+                const int o = k & cross;  // corner k's block, as an offset from corner 0's
+                s[k] = voxel(m, o ? ld_map<NC>(L + o - 1) : slot, vx, vy, vz, v);
+                ok &= v;
+            }
         }
         return ok;
-    }
-
-    // corners across block boundaries when corner 0's block is not allocated:
-    // one lookup per distinct block
-    static __device__ __forceinline__ bool load8_general(const DevMap& m, Ray& r, const Corners& c, float* s)
-    {
-        bool ok = true;
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-            const int vx = (k & 1) ? c.x1 : c.x0, vy = (k & 2) ? c.y1 : c.y0, vz = (k & 4) ? c.z1 : c.z0;
-            bool v;
-            s[k] = voxel(m, block_of(m, r, vox2blk(vx), vox2blk(vy), vox2blk(vz)), vx, vy, vz, v);
-            ok &= v;
-        }
-        return ok;
-    }
-
-    static __device__ __forceinline__ float interp(const DevMap& m, Ray& r, float3 p, bool& valid)
-    {
-        const Corners c = corners(p);
-        float s[8];
-        const int slot = block_of(m, r, vox2blk(c.x0), vox2blk(c.y0), vox2blk(c.z0));
-        if (slot >= 0) {
-            valid = c.inner() ? load8(m, slot, c, s) == 0xffu : load8_linked(m, slot, c, s);
-        } else if (c.inner()) {
-            valid = false;
-#pragma unroll
-            for (int k = 0; k < 8; ++k) s[k] = 1.f;
-        } else {
-            valid = load8_general(m, r, c, s);
-        }
-        return lerp8(s, c.ax, c.ay, c.az);
     }
 
     // Every 1-voxel step inside the unallocated block (bx, by, bz) reads
     // (1.0, invalid): jump to the first step past the block's exit (at least
     // one step). Exit faces: +8 where the ray runs up (and +0), +0 where it
     // runs down (and -0), so a zero component gives an infinite distance.
-    static __device__ __forceinline__ void empty_jump(Ray& r, int bx, int by, int bz)
+    // One multiply-add, rounded down, gives a coordinate's block in the narrow
+    // form and a second one its exit face (both exact), so that a jump is some
+    // 20 multiply-adds and 4 operations of the half-rate ALU, which bounds this
+    // loop: with the faces from the integer codes it took 22 of them.
+    static __device__ __forceinline__ void empty_jump(Ray& r)
     {
-        const float tx = ((float)(bx * 8 + (signbit(r.dir.x) ? 0 : 8)) - r.res.x) * r.inv.x;
-        const float ty = ((float)(by * 8 + (signbit(r.dir.y) ? 0 : 8)) - r.res.y) * r.inv.y;
-        const float tz = ((float)(bz * 8 + (signbit(r.dir.z) ? 0 : 8)) - r.res.z) * r.inv.z;
+        auto face = [](float p, float d) {
+            if constexpr (WIDE) return __int2float_rn((fl(p) & ~7) + (signbit(d) ? 0 : 8));
+            else return __fmaf_rn(__fmaf_rd(p, 0.125f, kFloorAdd), 8.f, (signbit(d) ? 0.f : 8.f) - 8.f * kFloorAdd);
+        };
+        const float tx = __fmul_rn(__fsub_rn(face(r.res.x, r.dir.x), r.res.x), r.inv.x);
+        const float ty = __fmul_rn(__fsub_rn(face(r.res.y, r.dir.y), r.res.y), r.inv.y);
+        const float tz = __fmul_rn(__fsub_rn(face(r.res.z, r.dir.z), r.res.z), r.inv.z);
         const float t = fminf(fminf(tx, ty), tz);  // fminf drops the NaN of 0 * inf
-        const float k = fmaxf(1.f, ceilf(t - 1e-3f));
+        float up;
+        if constexpr (WIDE) up = ceilf(t - 1e-3f);
+        else up = __fsub_rn(__fadd_ru(__fsub_rn(t, 1e-3f), kFloorAdd), kFloorAdd);  // the same, t < 2^22
+        const float k = fmaxf(1.f, up);
         r.res = fma3(k, r.dir, r.res);
         r.dist_s = __fadd_rn(r.dist_s, k);
     }
 
     // Start a ray at pixel (x, y); false when it finishes at once (tile with
     // no allocated block: written as a miss).
-    static __device__ __forceinline__ bool init(const MapView& v, Ray& r, int mi, int x, int y)
+    static __device__ __forceinline__ bool init(const MapView& v, Ray& r, int x, int y)
     {
         const RenderOut& o = v.out;
         const CamParams& c = v.cam;
@@ -243,7 +257,7 @@ struct March {
         r.dist_lim = dist_e;
         if (o.mode == 0) {
             // ray length (voxels) is proportional to camera depth along a ray
-            const float g = dist_e / kMaxDepth;
+            const float g = div_exact(dist_e, kMaxDepth, 1.f / kMaxDepth);
             const float k0 = floorf(g * zn - dist0) - 2.f;
             if (k0 > 0.f) {
                 r.res = fma3(k0, r.dir, r.res);
@@ -258,49 +272,96 @@ struct March {
             // instrumented run found every skipped block empty; positions agree
             // with the lookup path to float rounding).
             const float lim = g * zn - 1.f;
-            while (r.dist_s < lim && r.dist_s < r.dist_lim)
-                empty_jump(r, vox2blk(__float2int_rz(floorf(r.res.x))), vox2blk(__float2int_rz(floorf(r.res.y))),
-                           vox2blk(__float2int_rz(floorf(r.res.z))));
+            while (r.dist_s < lim && r.dist_s < r.dist_lim) empty_jump(r);
         }
-        r.mi = mi;
         r.x = x;
         r.y = y;
         r.sdf = 1.f;
         r.valid = false;
-        r.cbx = r.obx = INT_MIN;
-        r.cblk = r.oblk = -1;
+        r.cx = r.cy = r.cz = INT_MIN;  // a region of its own: no sample's codes have this top bit
+        r.cmask = 7;
+        r.cblk = -1;
+        r.bits = 0ull;
         return true;
     }
 
-    // First half of a loop iteration: the key of the block the sample at res
-    // falls in when that block is not the ray's current one and not its
-    // cached second block (kEmptyKey otherwise: no lookup needed). The block
-    // the ray leaves becomes the cached second block: the refinement step
-    // after the zero crossing steps back by up to half a truncation band, and
-    // at 640x480 / 5 mm it lands in that block on 27 % of rays (69 % stay in
-    // the current block; an oracle count over 3.1 M crossings).
-    static __device__ __forceinline__ unsigned long long lookup_key(Ray& r, const Cell& c)
+    // Bits in which floor codes (ix, iy, iz) differ from the last looked-up
+    // voxel's: none above r.cmask, and they lie in the same settled region.
+    static __device__ __forceinline__ int moved(const Ray& r, int ix, int iy, int iz)
     {
-        const int bx = vox2blk(c.x0), by = vox2blk(c.y0), bz = vox2blk(c.z0);
-        if (bx == r.cbx && by == r.cby && bz == r.cbz) return kEmptyKey;
-        const bool second = bx == r.obx && by == r.oby && bz == r.obz;
-        const int oblk = r.oblk;
-        r.obx = r.cbx;
-        r.oby = r.cby;
-        r.obz = r.cbz;
-        r.oblk = r.cblk;
-        r.cbx = bx;
-        r.cby = by;
-        r.cbz = bz;
-        if (second) {
-            r.cblk = oblk;
-            return kEmptyKey;
+        return (ix ^ r.cx) | (iy ^ r.cy) | (iz ^ r.cz);
+    }
+
+    // Looks the voxel up: the largest empty cube the occupancy words show
+    // around it, or its block's slot. Within the brick of the last lookup its
+    // word is at hand and an empty block needs no read; in a new brick the
+    // three reads do not depend on one another.
+    static __device__ __forceinline__ void settle(const DevMap& m, Ray& r, int ix, int iy, int iz, bool same_brick)
+    {
+        const int bx = ix >> 3, by = iy >> 3, bz = iz >> 3;
+        const int bit = grid_bit(bx, by, bz);
+        const int brick = grid_brick(m, bx, by, bz);
+        const unsigned long long* cell = m.grid + ((size_t)brick * 64 + bit);
+        unsigned long long e = 0ull;
+        r.cmask = 7;
+        if (same_brick) {
+            if ((r.bits >> bit) & 1ull) e = ld_map<NC>(cell);
+        } else {
+            const unsigned long long above = ld_map<NC>(m.occ2 + grid_region(m, bx, by, bz));
+            r.bits = ld_map<NC>(m.occ + brick);
+            e = ld_map<NC>(cell);
+            if (r.bits == 0ull) r.cmask = above == 0ull ? 127 : 31;
         }
-        if (!coord_ok(bx, by, bz)) {
-            r.cblk = -1;
-            return kEmptyKey;
+        r.cblk = slot_of(m, e, ix, iy, iz);
+    }
+
+    // Ray distance up to which a ray at res is certain to stay in its empty
+    // cube: the exit distance less a margin for the rounding of the jumps'
+    // positions. (Wide views look at every position instead.)
+    static __device__ __forceinline__ float run_limit(const Ray& r, float slack)
+    {
+        if constexpr (WIDE) return r.dist_s;
+        auto exit = [&r](int i, float p, float d, float inv) {
+            return (ff(i & ~r.cmask) + (signbit(d) ? 0.f : (float)(r.cmask + 1)) - p) * inv;
+        };
+        const float t = fminf(fminf(exit(r.cx, r.res.x, r.dir.x, r.inv.x), exit(r.cy, r.res.y, r.dir.y, r.inv.y)),
+                              exit(r.cz, r.res.z, r.dir.z, r.inv.z));
+        return fminf(r.dist_lim, r.dist_s + t - slack);
+    }
+
+    // First half of a loop iteration: from the sample at res towards the first
+    // one in an allocated block (slot r.cblk, its voxel in cx, cy, cz), over up
+    // to kSeek empty cubes. Each unallocated block on the way reads (1.0,
+    // invalid) and is jumped over, one jump a block as in the reference's
+    // lattice, but looked up only once per empty cube. kSeek bounds how long
+    // the rays of the warp that are in a block wait for those that cross empty
+    // space, to about the time of a sample: at grazing views every iteration
+    // has some ray with a long way to go, and a warp whose iterations all
+    // waited for it took 438 turns of the jump loop where no ray of it made
+    // more than 45 jumps.
+    static constexpr int kSeek = 2;
+    enum Seek { kOut, kBlock, kOnTheWay };  // the ray's range ended, in a block, neither yet
+
+    static __device__ __forceinline__ Seek seek(const MapView& v, Ray& r)
+    {
+#pragma unroll 1
+        for (int n = 0; n <= kSeek; ++n) {
+            if (!(r.dist_s < r.dist_lim)) return kOut;
+            if (n == kSeek) break;
+            const int ix = fl(r.res.x), iy = fl(r.res.y), iz = fl(r.res.z);
+            const int d = moved(r, ix, iy, iz);
+            r.cx = ix;
+            r.cy = iy;
+            r.cz = iz;
+            if (d & ~r.cmask) settle(v.m, r, ix, iy, iz, !(d & ~31));
+            if (r.cblk >= 0) return kBlock;
+            const float run = run_limit(r, v.out.slack);
+            do empty_jump(r);
+            while (r.dist_s < run);
+            r.sdf = 1.f;
+            r.valid = false;
         }
-        return pack_key(bx, by, bz);
+        return kOnTheWay;
     }
 
     // An unobserved voxel of an allocated block reads (1.0, invalid), and the
@@ -328,10 +389,10 @@ struct March {
         for (int k = 0; k < kRunAhead; ++k) {
             q = fma3(1.f, r.dir, q);
             ds = __fadd_rn(ds, 1.f);
-            const Cell c = cell(q);
-            ok[k] = ds < r.dist_lim && vox2blk(c.x0) == r.cbx && vox2blk(c.y0) == r.cby && vox2blk(c.z0) == r.cbz;
+            const int ix = fl(q.x), iy = fl(q.y), iz = fl(q.z);
+            ok[k] = ds < r.dist_lim && !(moved(r, ix, iy, iz) & ~7);
             w[k] = Word();
-            if (ok[k]) w[k] = ld_map<NC>(blk + local_idx(c.x0, c.y0, c.z0));
+            if (ok[k]) w[k] = ld_map<NC>(blk + at(ix, iy, iz));
         }
         int n = 1;  // samples consumed: this one, then the leading unobserved ones ahead
         bool run = true;
@@ -348,45 +409,26 @@ struct March {
         r.valid = false;
     }
 
-    // Second half: one iteration of the reference loop with the sample's block
-    // (r.cblk) known; true when the ray leaves the loop.
-    static __device__ __forceinline__ bool advance(const MapView& v, Ray& r, const Cell& p)
+    // Second half: one iteration of the reference loop at the sample at res,
+    // voxel (cx, cy, cz) of block r.cblk; true when the ray leaves the loop.
+    // The sample and the link its corners may need are read together, the
+    // other corners after it.
+    static __device__ __forceinline__ bool advance(const MapView& v, Ray& r)
     {
         const DevMap& m = v.m;
-        const int bx = r.cbx, by = r.cby, bz = r.cbz;
-        if (r.cblk < 0) {
-            empty_jump(r, bx, by, bz);
-            r.sdf = 1.f;
-            r.valid = false;
-            return false;
-        }
+        const Corners c = corners(r.res, r.cx, r.cy, r.cz);
+        const int cross = c.cross();
+        const Word w0 = ld_map<NC>(Layout<FMT>::words(m, r.cblk) + at(c.x0, c.y0, c.z0));  // read_sdf at floor(res)
+        const int far = far_slot(m, r.cblk, cross);
         bool valid;
-        float sdf = voxel(m, r.cblk, p.x0, p.y0, p.z0, valid);  // read_sdf at floor(res)
+        float sdf = value(w0, valid);
         if (!valid) {
             unobserved_run(v, r);
             return false;
         }
         if (sdf <= 0.5f && sdf >= -0.5f) {
             float s[8];
-            const Corners c = corners(r.res);  // c.x0 == p.x0 (same position)
-            if (c.inner()) {
-                // corner 0 is the sample just read; the other 7 are independent
-                // loads (loading all 8 with every sample was measured slower)
-                const Word* w = Layout<FMT>::words(m, r.cblk) + local_idx(c.x0, c.y0, c.z0);
-                const Word w1 = ld_map<NC>(w + 1), w2 = ld_map<NC>(w + 8), w3 = ld_map<NC>(w + 9), w4 = ld_map<NC>(w + 64);
-                const Word w5 = ld_map<NC>(w + 65), w6 = ld_map<NC>(w + 72), w7 = ld_map<NC>(w + 73);
-                bool v;
-                s[0] = sdf;
-                s[1] = value(w1, v); valid &= v;
-                s[2] = value(w2, v); valid &= v;
-                s[3] = value(w3, v); valid &= v;
-                s[4] = value(w4, v); valid &= v;
-                s[5] = value(w5, v); valid &= v;
-                s[6] = value(w6, v); valid &= v;
-                s[7] = value(w7, v); valid &= v;
-            } else {
-                valid = load8_linked(m, r.cblk, c, s);
-            }
+            valid = corners8(m, r.cblk, far, cross, c, w0, s);
             sdf = lerp8(s, c.ax, c.ay, c.az);
         }
         r.sdf = sdf;
@@ -400,32 +442,40 @@ struct March {
 
     // After the loop: two refinement steps when the zero crossing was found
     // (ray_tracing.cu:381-393), then the camera-frame vertex or a miss. The
-    // first step is taken here; the block of the interpolation's first corner
-    // becomes the ray's current block, and its key is returned when it is
-    // neither the block the ray is in nor the one it came from (4 % of
-    // crossings at 640x480 / 5 mm) and has to be looked up.
-    static __device__ __forceinline__ unsigned long long refine_key(const MapView& v, Ray& r)
-    {
-        if (!(r.sdf <= 0.f)) return kEmptyKey;
-        r.res = fma3(__fmul_rn(r.sdf, v.out.rts), r.dir, r.res);
-        return lookup_key(r, cell(r.res));
-    }
-
-    // The rest, with the current block's slot (r.cblk) known.
+    // first step lands in the block the ray is in on 69 % of crossings and in
+    // the one before on 27 % (640x480 / 5 mm, an oracle count).
     static __device__ __forceinline__ void finish(const MapView& v, Ray& r)
     {
         const RenderOut& o = v.out;
         bool found = false;
         if (r.sdf <= 0.f) {
-            bool valid;
-            const float s = interp(v.m, r, r.res, valid);  // first corner's block: r.cblk
+            r.res = fma3(__fmul_rn(r.sdf, o.rts), r.dir, r.res);
+            const int ix = fl(r.res.x), iy = fl(r.res.y), iz = fl(r.res.z);
+            int slot = r.cblk;
+            if (moved(r, ix, iy, iz) & ~7) slot = slot_of(v.m, entry(v.m, ix, iy, iz), ix, iy, iz);
+            bool valid = false;
+            const Corners c = corners(r.res, ix, iy, iz);
+            const int cross = c.cross();
+            float e[8];
+            if (slot >= 0) {
+                const Word w0 = ld_map<NC>(Layout<FMT>::words(v.m, slot) + at(ix, iy, iz));
+                valid = corners8(v.m, slot, far_slot(v.m, slot, cross), cross, c, w0, e);
+            } else {  // corner 0's block is not allocated: the read is invalid, its value still counts
+#pragma unroll
+                for (int k = 0; k < 8; ++k) {
+                    const int vx = (k & 1) ? c.x1 : c.x0, vy = (k & 2) ? c.y1 : c.y0, vz = (k & 4) ? c.z1 : c.z0;
+                    bool ok;
+                    e[k] = k & cross ? voxel(v.m, slot_of(v.m, entry(v.m, vx, vy, vz), vx, vy, vz), vx, vy, vz, ok) : 1.f;
+                }
+            }
+            const float s = lerp8(e, c.ax, c.ay, c.az);
             r.res = fma3(__fmul_rn(s, o.rts), r.dir, r.res);
             found = valid;
         }
         float4 out;
         if (found) {
-            const float3 q = xf_apply(v.Ti, __fdiv_rn(r.res.x, o.vsinv), __fdiv_rn(r.res.y, o.vsinv),
-                                      __fdiv_rn(r.res.z, o.vsinv));
+            const float3 q = xf_apply(v.Ti, div_exact(r.res.x, o.vsinv, o.vsinvRcp), div_exact(r.res.y, o.vsinv, o.vsinvRcp),
+                                      div_exact(r.res.z, o.vsinv, o.vsinvRcp));
             out = make_float4(q.x, q.y, q.z, 1.f);
         } else {
             const float qnan = __int_as_float(0x7fffffff);
@@ -435,103 +485,30 @@ struct March {
     }
 };
 
-// Per-warp block cache in shared memory (64 direct-mapped entries), shared by
-// the 32 rays of the warp's tile and kept across the warp's tiles of one map.
-// Called by all lanes together: lanes that miss look their block up once per
-// distinct key (__match_any_sync), and each cache line gets one writer, so an
-// entry's key and slot always belong together.
-constexpr int kWarpCache = 64;
-
-template <bool NC>
-__device__ __forceinline__ int warp_lookup(const DevMap& m, unsigned long long key, unsigned long long* wkey,
-                                           int* wslot, int lane)
+// One warp marches tile q of the nt tiles of a map (q counts in the order the
+// tiles are handed out).
+template <int FMT, bool NC, bool WIDE>
+__device__ __forceinline__ void march_tile(const MapView& v, int q, int nt, int order, int tw, int lane)
 {
-    const unsigned full = 0xffffffffu;
-    const bool need = key != kEmptyKey;
-    if (!__ballot_sync(full, need)) return -1;
-    const unsigned idx = (unsigned)((key * 0x9E3779B97F4A7C15ull) >> 58);
-    int slot = -1;
-    bool miss = false;
-    if (need) {
-        if (wkey[idx] == key) slot = wslot[idx];
-        else miss = true;
-    }
-    if (__ballot_sync(full, miss)) {
-        const unsigned grp = __match_any_sync(full, miss ? key : kEmptyKey);
-        const int leader = __ffs(grp) - 1;
-        int s = -1;
-        if (miss && lane == leader) {
-            const int3 b = unpack_key(key);
-            s = hash_find<NC>(m, b.x, b.y, b.z);
-        }
-        s = __shfl_sync(full, s, leader);
-        if (miss) slot = s;
-        const bool writer = miss && lane == leader;
-        const unsigned ig = __match_any_sync(full, writer ? (int)idx : -1);
-        __syncwarp();
-        if (writer && lane == __ffs(ig) - 1) {
-            wkey[idx] = key;
-            wslot[idx] = s;
-        }
-        __syncwarp();
-    }
-    return slot;
-}
-
-// One warp marches tile q of the nt tiles of map mi (q counts in the order
-// the tiles are handed out). The warp's block cache must hold blocks of this
-// map only.
-template <int FMT, bool NC>
-__device__ __forceinline__ void march_tile(const MapView& v, int mi, int q, int nt, int order, int tw,
-                                           unsigned long long* wkey, int* wslot, int lane)
-{
-    typedef March<FMT, NC> M;
-    typedef typename M::Cell Cell;
-    const unsigned full = 0xffffffffu;
+    typedef March<FMT, NC, WIDE> M;
     // the map's q-th tile in the requested order (row-major tile index t):
     // 0 bottom rows first, 1 top rows first, 2 alternating from both ends
     const int t = order == 1 ? q : order == 2 ? ((q & 1) ? nt - 1 - (q >> 1) : (q >> 1)) : nt - 1 - q;
     const int tx = (v.cam.W + tw - 1) / tw;
     const int x = (t % tx) * tw + (lane % tw), y = (t / tx) * (32 / tw) + (lane / tw);
     Ray r;
-    bool live = x < v.cam.W && y < v.cam.H && M::init(v, r, mi, x, y);
-    const bool started = live;
-    // warp-synchronous march: every lane reaches the shared lookup each
-    // iteration; finished lanes idle until the tile is done, then all
-    // finish together
-    while (__ballot_sync(full, live)) {
-        Cell c;
-        unsigned long long key = kEmptyKey;
-        if (live) {
-            if (!(r.dist_s < r.dist_lim)) live = false;
-            else {
-                c = M::cell(r.res);
-                key = M::lookup_key(r, c);
-            }
-        }
-        const int slot = warp_lookup<NC>(v.m, key, wkey, wslot, lane);
-        if (key != kEmptyKey) r.cblk = slot;
-        if (live && M::advance(v, r, c)) live = false;
+    const bool started = x < v.cam.W && y < v.cam.H && M::init(v, r, x, y);
+    // warp-synchronous march: the lanes meet at both halves of an iteration,
+    // so their sample and corner reads are issued together; finished lanes
+    // idle until the tile is done, then all finish together
+    bool live = started;
+    while (__any_sync(0xffffffffu, live)) {
+        int at = M::kOut;
+        if (live) at = M::seek(v, r);
+        __syncwarp();
+        live = at == M::kOnTheWay || (at == M::kBlock && !M::advance(v, r));
     }
-    // the first refinement step's block, looked up per lane when the ray's
-    // two cached blocks miss it (measured faster on the batched step than the
-    // same lookup through the warp's block cache)
-    if (started) {
-        const unsigned long long key = M::refine_key(v, r);
-        if (key != kEmptyKey) {
-            const int3 b = unpack_key(key);
-            r.cblk = hash_find<NC>(v.m, b.x, b.y, b.z);
-        }
-        M::finish(v, r);
-    }
-}
-
-// Empty the warp's block cache (all lanes of the warp).
-__device__ __forceinline__ void warp_cache_clear(unsigned long long* wkey, int lane)
-{
-    wkey[lane] = kEmptyKey;
-    wkey[lane + 32] = kEmptyKey;
-    __syncwarp();
+    if (started) M::finish(v, r);
 }
 
 }  // namespace vmapb

@@ -19,7 +19,7 @@
 //   * inside an unallocated block, where the reference reads "invalid, 1.0"
 //     and steps 1 voxel at a time, the steps up to the block's exit are taken
 //     as one integer jump;
-//   * block lookups are cached per thread.
+//   * whole empty cubes of blocks are crossed without lookups (raymarch.cu).
 // The ray marcher itself lives in raymarch.cu.
 #include "stages.cuh"
 

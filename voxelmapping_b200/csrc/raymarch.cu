@@ -11,9 +11,17 @@
 //     and steps one voxel at a time, the steps up to the block's exit are
 //     taken as one integer jump; before the tile's nearest allocated block
 //     these jumps need no lookup and are taken when the ray starts;
-//   * when the 8 trilinear corners sit in the current block, the 7 besides
-//     the centre sample are read with independent loads (no lookups between);
-//   * hash lookups are cached per ray (current block + one neighbour).
+//   * whole empty cubes of blocks are recognised from the block grid's
+//     occupancy words, so that the jumps inside one need no lookup either;
+//   * the trilinear corners of all rays of a warp are read together, whether
+//     they lie in one block or two.
+// What bounds it: the instructions (a third to a half of them on the ALU pipe,
+// which runs at half rate: at 640x480 the kernel issues 70 % of the time while
+// all its warps run) and, in scenes seen at grazing angles, the slowest tiles'
+// latency. Against a lookup per block through a warp-shared cache and the hash
+// table, event time of the launch, three rooms each: 48 -> 33 us at 160x120 /
+// 16 mm, 63 -> 42 at 320x240 / 8 mm, 96 -> 69 at 640x480 / 5 mm, 293 -> 234 at
+// 1280x720 / 4 mm, 320 -> 129 for an 800x600 full march (raycast_mode 1).
 //
 // Scheduling: the kernel is persistent. Each warp takes 8x4-pixel tiles from
 // one device-side queue shared by every map of the batch until it runs dry.
@@ -27,15 +35,11 @@
 
 namespace vmapb {
 
-// 4 CTAs per SM (at most 64 registers) measured faster than the 3 that 76
-// registers allow: latency hiding outweighs a small register spill.
-template <class V, int FMT>
-__global__ void __launch_bounds__(256, 4) raycast_kernel(const __grid_constant__ V views, int order, int tw)
+template <class V, int FMT, bool WIDE>
+__device__ __forceinline__ void raycast_tiles(const V& views, int order, int tw)
 {
     stage_entry();
     __shared__ int pre[kMaxBatch + 1];
-    __shared__ unsigned long long s_wkey[8][kWarpCache];
-    __shared__ int s_wslot[8][kWarpCache];
     map_prefix(views, [tw](const MapView& v) { return ray_tiles(v, tw); }, pre);
     // the z-range pass before this launch linked every allocated block of the
     // maps it renders
@@ -45,62 +49,70 @@ __global__ void __launch_bounds__(256, 4) raycast_kernel(const __grid_constant__
     const int nmaps = views.count();
     const int total = pre[nmaps];
     const int lane = threadIdx.x & 31;
-    unsigned long long* wkey = s_wkey[threadIdx.x >> 5];
-    int* wslot = s_wslot[threadIdx.x >> 5];
-    int wmap = -1;  // map whose blocks the warp cache holds
-    for (;;) {
-        int item = 0;
-        if (lane == 0) item = (int)atomicAdd(views.queue, 1u);
-        item = __shfl_sync(0xffffffffu, item, 0);
-        if (item >= total) break;
+    // a warp's first tile is its own number (consecutive tiles on different
+    // SMs), the others come from the queue
+    const int warps = (int)(gridDim.x * (blockDim.x >> 5));
+    int item = (int)((threadIdx.x >> 5) * gridDim.x + blockIdx.x);
+    while (item < total) {
         const int mi = map_of(pre, nmaps, item);
-        if (mi != wmap) {
-            warp_cache_clear(wkey, lane);
-            wmap = mi;
-        }
-        march_tile<FMT, true>(views[mi], mi, item - pre[mi], pre[mi + 1] - pre[mi], order, tw, wkey, wslot, lane);
+        march_tile<FMT, true, WIDE>(views[mi], item - pre[mi], pre[mi + 1] - pre[mi], order, tw, lane);
+        if (lane == 0) item = warps + (int)atomicAdd(views.queue, 1u);
+        item = __shfl_sync(0xffffffffu, item, 0);
     }
 }
 
+// 4 CTAs per SM (at most 64 registers) measured faster than the 3 that 76
+// registers allow: latency hiding outweighs a small register spill.
 template <class V, int FMT>
+__global__ void __launch_bounds__(256, 4) raycast_kernel(const __grid_constant__ V views, int order, int tw)
+{
+    raycast_tiles<V, FMT, false>(views, order, tw);
+}
+
+// The same for launches with a view whose rays leave the narrow range.
+template <class V, int FMT>
+__global__ void __launch_bounds__(256, 3) march_wide_kernel(const __grid_constant__ V views, int order, int tw)
+{
+    raycast_tiles<V, FMT, true>(views, order, tw);
+}
+
+template <class V, int FMT, bool WIDE>
 static cudaError_t raycast_persistent(const V& views, const Launcher& l, cudaStream_t s)
 {
+    static void (*const kernel)(const V, int, int) = WIDE ? march_wide_kernel<V, FMT> : raycast_kernel<V, FMT>;
     // resident CTAs per SM of this instantiation at 128 and 256 threads (a
     // static initialiser runs once, thread-safely, on the first launch)
-    static const int occ[2] = {[] {
-                                   int o = 0;
-                                   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, raycast_kernel<V, FMT>, 128,
-                                                                                     0) != cudaSuccess || o < 1)
-                                       o = 1;
-                                   return o;
-                               }(),
-                               [] {
-                                   int o = 0;
-                                   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, raycast_kernel<V, FMT>, 256,
-                                                                                     0) != cudaSuccess || o < 1)
-                                       o = 1;
-                                   return o;
-                               }()};
+    auto fits = [](int threads) {
+        int o = 0;
+        return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, kernel, threads, 0) != cudaSuccess || o < 1 ? 1 : o;
+    };
+    static const int occ[2] = {fits(128), fits(256)};
     const int threads = l.rayThreads == 128 ? 128 : 256;
     const int fit = occ[threads == 256];
     // CTAs beyond those resident would only start once others finish: cap at occupancy
     const int per_sm = l.raycast > 0 && l.raycast < fit ? l.raycast : fit;
-    return launch_stage<V>(raycast_kernel<V, FMT>, stage_grid(l, per_sm), threads, s, views, l.tileOrder, l.tileW);
+    return launch_stage<V>(kernel, stage_grid(l, per_sm), threads, s, views, l.tileOrder, l.tileW);
+}
+
+template <class V, int FMT>
+static cudaError_t raycast_format(const V& views, bool wide, const Launcher& l, cudaStream_t s)
+{
+    return wide ? raycast_persistent<V, FMT, true>(views, l, s) : raycast_persistent<V, FMT, false>(views, l, s);
 }
 
 template <class V>
-cudaError_t launch_raycast(const V& views, int fmt, const Launcher& l, cudaStream_t s)
+cudaError_t launch_raycast(const V& views, int fmt, bool wide, const Launcher& l, cudaStream_t s)
 {
     switch (fmt) {
-    case VMAP_VOXEL_REF: return raycast_persistent<V, VMAP_VOXEL_REF>(views, l, s);
-    case VMAP_VOXEL_F32: return raycast_persistent<V, VMAP_VOXEL_F32>(views, l, s);
-    case VMAP_VOXEL_F16: return raycast_persistent<V, VMAP_VOXEL_F16>(views, l, s);
-    case VMAP_VOXEL_I16: return raycast_persistent<V, VMAP_VOXEL_I16>(views, l, s);
+    case VMAP_VOXEL_REF: return raycast_format<V, VMAP_VOXEL_REF>(views, wide, l, s);
+    case VMAP_VOXEL_F32: return raycast_format<V, VMAP_VOXEL_F32>(views, wide, l, s);
+    case VMAP_VOXEL_F16: return raycast_format<V, VMAP_VOXEL_F16>(views, wide, l, s);
+    case VMAP_VOXEL_I16: return raycast_format<V, VMAP_VOXEL_I16>(views, wide, l, s);
     default: return cudaErrorInvalidValue;
     }
 }
 
-template cudaError_t launch_raycast<OneView>(const OneView&, int, const Launcher&, cudaStream_t);
-template cudaError_t launch_raycast<ManyViews>(const ManyViews&, int, const Launcher&, cudaStream_t);
+template cudaError_t launch_raycast<OneView>(const OneView&, int, bool, const Launcher&, cudaStream_t);
+template cudaError_t launch_raycast<ManyViews>(const ManyViews&, int, bool, const Launcher&, cudaStream_t);
 
 }  // namespace vmapb

@@ -62,6 +62,7 @@ __device__ void hash_insert_slot(const DevMap& m, unsigned long long key, unsign
             if (cur == kEmptyKey) cur = atomicCAS(&s[i].x, kEmptyKey, key);
             if (cur == kEmptyKey) {
                 s[i].y = (unsigned long long)slot;
+                grid_insert(m, c.x, c.y, c.z, slot);
                 return;
             }
             if (cur == key) {
@@ -95,6 +96,12 @@ __global__ void clear_slots_kernel(DevMap m)
     const size_t n = (size_t)m.nBucket * kSlots;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
         m.slots[i] = make_ulonglong2(kEmptyKey, ~0ull);
+    const size_t cells = grid_cells(m.capacity);
+    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < cells; i += (size_t)gridDim.x * blockDim.x) {
+        m.grid[i] = 0ull;
+        if (i < cells / 64) m.occ[i] = 0ull;
+        if (i < cells / 4096) m.occ2[i] = 0ull;
+    }
 }
 
 int sm_count()
@@ -200,7 +207,7 @@ vmap_status vmap_snapshot_load(vmap_map* map, const void* src, uint64_t bytes, v
     if (st.allocated_blocks > n)
         SNAP_CK(cudaMemsetAsync(m.pool + (size_t)n * m.blockBytes, 0, (size_t)(st.allocated_blocks - n) * m.blockBytes, s));
     SNAP_CK(cudaMemsetAsync(m.ctr, 0, C_UNKNOWN * sizeof(unsigned), s));
-    clear_slots_kernel<<<grid_for((size_t)m.nBucket * kSlots), 256, 0, s>>>(m);
+    clear_slots_kernel<<<grid_for((size_t)m.nBucket * kSlots + grid_cells(m.capacity)), 256, 0, s>>>(m);
     SNAP_CK(cudaGetLastError());
     if (n) {
         SNAP_CK(cudaMemcpyAsync(m.blockKeys, p + h.keys_offset, 8ull * n, cudaMemcpyDefault, s));

@@ -286,10 +286,10 @@ __device__ __forceinline__ void link_task(const DevMap& m, int t)
     const int k = 1 + (t % 14) / 2, dx = k & 1, dy = (k >> 1) & 1, dz = (k >> 2) & 1;
     const int3 b = unpack_key(m.blockKeys[slot]);
     if (t & 1) {  // a backward neighbour's link to this block
-        const int e = hash_find<NC>(m, b.x - dx, b.y - dy, b.z - dz);
+        const int e = block_find<NC>(m, b.x - dx, b.y - dy, b.z - dz);
         if (e >= 0) m.nbr[7 * (size_t)e + k - 1] = slot;
     } else {
-        m.nbr[7 * (size_t)slot + k - 1] = hash_find<NC>(m, b.x + dx, b.y + dy, b.z + dz);
+        m.nbr[7 * (size_t)slot + k - 1] = block_find<NC>(m, b.x + dx, b.y + dy, b.z + dz);
     }
 }
 

@@ -143,8 +143,6 @@ template <int FMT>
 __global__ void __launch_bounds__(256, 4) step_kernel(const __grid_constant__ ManyViews views, StepSched* S,
                                                        int order, int tw, unsigned long long stallNs)
 {
-    __shared__ unsigned long long s_wkey[8][kWarpCache];
-    __shared__ int s_wslot[8][kWarpCache];
     __shared__ unsigned long long s_set[8][kWarpSet];
     const unsigned full = 0xffffffffu;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -159,14 +157,13 @@ __global__ void __launch_bounds__(256, 4) step_kernel(const __grid_constant__ Ma
     // scheduler state of each warp, kept in shared memory rather than in
     // registers across the item bodies: lane 0's ring cursor, the task the
     // warp takes items from, its item count and aux value, the warp's items
-    // of that task not yet counted done, the item in hand, and the map whose
-    // blocks the warp's block cache holds
+    // of that task not yet counted done, and the item in hand
     __shared__ int s_state[8][8];
     int* st = s_state[wid];
-    enum { H, CUR, TOTAL, AUX, UNCOUNTED, ITEM, WMAP };
+    enum { H, CUR, TOTAL, AUX, UNCOUNTED, ITEM };
     if (lane == 0) {
         st[H] = st[TOTAL] = st[AUX] = st[UNCOUNTED] = st[ITEM] = 0;
-        st[CUR] = st[WMAP] = -1;
+        st[CUR] = -1;
     }
     __syncwarp();
     for (;;) {
@@ -248,11 +245,7 @@ __global__ void __launch_bounds__(256, 4) step_kernel(const __grid_constant__ Ma
             break;
         }
         case ST_RAYCAST:
-            if (mi != st[WMAP]) {
-                warp_cache_clear(s_wkey[wid], lane);  // ends with __syncwarp
-                if (lane == 0) st[WMAP] = mi;
-            }
-            march_tile<FMT, false>(v, mi, i, st[TOTAL], order, tw, s_wkey[wid], s_wslot[wid], lane);
+            march_tile<FMT, false, true>(v, i, st[TOTAL], order, tw, lane);
             break;
         default: {  // normals of a 32x8-pixel tile
             const int tx = (v.cam.W + 31) >> 5;

@@ -61,6 +61,12 @@ struct DevMap {
     // or -1 while that block is not allocated; set for the blocks below
     // ctr[C_LINKED] (all of them once a z-range pass has run)
     int* nbr;                      // capacity * 7
+    // block grid: a torus of 2^gridLog2 cells per axis over the block
+    // coordinates, in bricks of 4 x 4 x 4 cells (grid_cell)
+    unsigned long long* occ;       // one word per brick: bit set when a block was allocated in that cell
+    unsigned long long* occ2;      // one word per 4 x 4 x 4 bricks: bit set when the brick's word is not zero
+    unsigned long long* grid;      // one entry per cell (grid_entry)
+    int gridLog2;
     unsigned long long bucketMagic;  // ceil(2^64 / nBucket): remainder by multiplication
     int nBucket;
     int capacity;
@@ -82,6 +88,18 @@ __device__ __forceinline__ float3 xf_apply(const Xf& t, float v0, float v1, floa
     o.y = __fadd_rn(__fmaf_rn(t.m[1][0], v0, __fmul_rn(t.m[1][1], v1)), __fmaf_rn(t.m[1][2], v2, t.m[1][3]));
     o.z = __fadd_rn(__fmaf_rn(t.m[2][0], v0, __fmul_rn(t.m[2][1], v1)), __fmaf_rn(t.m[2][2], v2, t.m[2][3]));
     return o;
+}
+
+// a / b correctly rounded, given y = 1 / b correctly rounded: an approximate
+// quotient, one correction that makes it faithful, and one more, which by
+// Markstein's theorem (P. Markstein, "Computation of elementary functions on
+// the IBM RISC System/6000 processor", 1990) rounds it correctly as long as no
+// step underflows. Five multiply-adds; a divide costs about twice that.
+__device__ __forceinline__ float div_exact(float a, float b, float y)
+{
+    float q = __fmul_rn(a, y);
+    q = __fmaf_rn(__fmaf_rn(-b, q, a), y, q);
+    return __fmaf_rn(__fmaf_rn(-b, q, a), y, q);
 }
 
 // unproject (map_struct.h:189-194): ((ifx * (x - cx)) * z, (ify * (y - cy)) * z, z)
@@ -126,6 +144,65 @@ __device__ __forceinline__ int vox2blk(int v) { return v >> 3; }
 __device__ __forceinline__ int local_idx(int vx, int vy, int vz)
 {
     return ((vz & 7) << 6) | ((vy & 7) << 3) | (vx & 7);
+}
+
+// ---------------------------------------------------------------- block grid
+// A dense index beside the hash table for the block lookups of the ray
+// marcher. A cell's entry holds the first block allocated in it: slot (low 32
+// bits), coordinate tag (10 bits per axis above the cell bits) and kGridValid;
+// kGridShared marks a cell that a second block fell into, or one outside the
+// tag's range: only then does a lookup that does not match go on to the hash
+// table. A zero entry is an empty cell. One 8-byte read settles a lookup (a
+// hash bucket is 64 bytes at an unrelated address, and an absent block costs
+// one as well), neighbouring blocks share sectors, and the occupancy word of a
+// brick answers for 64 blocks at once, that of a region for 64 bricks: a ray
+// crosses empty space with a look at the words per empty cube (up to 16 blocks
+// wide) instead of one per block.
+// 8 cells per block of a large pool's surface share would be wasted on small
+// ones, so the side follows the capacity: 32 up to 2^12 blocks (0.26 MB), 64
+// up to 2^15 (2.1 MB), 128 above (17 MB; a 4 m room at 5 mm spans 100 blocks).
+constexpr unsigned kGridValid = 1u << 30, kGridShared = 1u << 31;  // in an entry's high word
+
+__host__ __device__ constexpr int grid_log2(int capacity)
+{
+    return capacity <= (1 << 12) ? 5 : capacity <= (1 << 15) ? 6 : 7;
+}
+
+// Voxel coordinates below which every block is within the tag's range and every
+// floor within 2^22, with room for a ray's last steps.
+__host__ __device__ constexpr double narrow_limit(int gridLog2) { return (4096 << gridLog2) - 1024; }
+
+__host__ __device__ constexpr size_t grid_cells(int capacity) { return (size_t)1 << (3 * grid_log2(capacity)); }
+
+// brick of block (x, y, z), region of 4 x 4 x 4 bricks, and the block's bit
+// within its brick (with x / 4, y / 4, z / 4: the brick's bit within its region)
+__device__ __forceinline__ int grid_brick(const DevMap& m, int x, int y, int z)
+{
+    const int l = m.gridLog2 - 2, mask = (1 << l) - 1;
+    return ((((z >> 2) & mask) << l | ((y >> 2) & mask)) << l) | ((x >> 2) & mask);
+}
+__device__ __forceinline__ int grid_region(const DevMap& m, int x, int y, int z)
+{
+    const int l = m.gridLog2 - 4, mask = (1 << l) - 1;
+    return ((((z >> 4) & mask) << l | ((y >> 4) & mask)) << l) | ((x >> 4) & mask);
+}
+__device__ __forceinline__ int grid_bit(int x, int y, int z) { return ((z & 3) << 4) | ((y & 3) << 2) | (x & 3); }
+
+// high word of block (x, y, z)'s entry: for blocks within the tag's range, from
+// the low bits of the coordinates alone
+__device__ __forceinline__ unsigned grid_tag_bits(const DevMap& m, int x, int y, int z)
+{
+    const int l = m.gridLog2;
+    return kGridValid | ((unsigned)(x >> l) & 1023u) << 20 | ((unsigned)(y >> l) & 1023u) << 10 | ((unsigned)(z >> l) & 1023u);
+}
+
+// the same for any block, 0 when its coordinates exceed the tag
+__device__ __forceinline__ unsigned grid_tag(const DevMap& m, int x, int y, int z)
+{
+    const int l = m.gridLog2;
+    const unsigned lim = 512u << l;
+    if ((unsigned)x + lim >= 2 * lim || (unsigned)y + lim >= 2 * lim || (unsigned)z + lim >= 2 * lim) return 0u;
+    return grid_tag_bits(m, x, y, z);
 }
 
 __device__ __forceinline__ bool coord_ok(int x, int y, int z)
@@ -256,6 +333,46 @@ __device__ __forceinline__ int hash_find(const DevMap& m, int bx, int by, int bz
     return -1;
 }
 
+// The block's slot through the grid (-1 when absent), given its brick and bit.
+template <bool NC>
+__device__ __forceinline__ int grid_find(const DevMap& m, int brick, int bit, int bx, int by, int bz)
+{
+    const unsigned long long e = ld_map<NC>(m.grid + ((size_t)brick * 64 + bit));
+    const unsigned hi = (unsigned)(e >> 32);
+    const unsigned tag = grid_tag(m, bx, by, bz);
+    if (tag && (hi & ~kGridShared) == tag) return (int)(unsigned)e;
+    return hi & kGridShared ? hash_find<NC>(m, bx, by, bz) : -1;
+}
+
+// hash_find's answer through the grid.
+template <bool NC = true>
+__device__ __forceinline__ int block_find(const DevMap& m, int bx, int by, int bz)
+{
+    return grid_find<NC>(m, grid_brick(m, bx, by, bz), grid_bit(bx, by, bz), bx, by, bz);
+}
+
+// Enter an allocated block into the grid.
+__device__ __forceinline__ void grid_insert(const DevMap& m, int bx, int by, int bz, unsigned slot)
+{
+    const int brick = grid_brick(m, bx, by, bz), bit = grid_bit(bx, by, bz);
+    const unsigned tag = grid_tag(m, bx, by, bz);
+    unsigned long long* cell = m.grid + ((size_t)brick * 64 + bit);
+    if (!tag || atomicCAS(cell, 0ull, (unsigned long long)tag << 32 | slot) != 0ull)
+        atomicOr(cell, (unsigned long long)kGridShared << 32);
+    if (atomicOr(m.occ + brick, 1ull << bit) == 0ull)
+        atomicOr(m.occ2 + grid_region(m, bx, by, bz), 1ull << grid_bit(bx >> 2, by >> 2, bz >> 2));
+}
+
+// Empty the cells of an allocated block (of every block: an empty grid).
+__device__ __forceinline__ void grid_clear(const DevMap& m, unsigned long long key)
+{
+    const int3 b = unpack_key(key);
+    const int brick = grid_brick(m, b.x, b.y, b.z);
+    m.grid[(size_t)brick * 64 + grid_bit(b.x, b.y, b.z)] = 0ull;
+    m.occ[brick] = 0ull;
+    m.occ2[grid_region(m, b.x, b.y, b.z)] = 0ull;
+}
+
 // Insert a block if absent (createBlock, map_struct.h:304-354, without its
 // lock: a compare-and-swap claims an empty slot, losers re-read). The winner
 // takes the next pool slot from a warp-aggregated bump counter, which hands
@@ -281,6 +398,7 @@ __device__ __forceinline__ void hash_insert(const DevMap& m, int bx, int by, int
                 if (slot < (unsigned)m.capacity) {
                     m.blockKeys[slot] = key;
                     s[i].y = (unsigned long long)slot;
+                    grid_insert(m, bx, by, bz, slot);
                 } else {
                     atomicOr(m.ctr + C_ERR, VMAP_FLAG_POOL_FULL);
                     atomicAdd(m.ctr + C_FAILED, 1u);
@@ -443,6 +561,9 @@ struct RenderOut {
     unsigned epoch;  // 1 .. 2^32 - 2
     int tilesX, tilesY;
     float vsinv;     // (float)(1.0 / (double)voxel_size)
+    float vsinvRcp;  // 1.f / vsinv
+    float slack;     // rounding of a ray position over a run of jumps, in voxels, with room to spare
+    int wide;        // rays may leave the narrow range of the ray marcher (March)
     float rts;       // truncation / voxel_size (raytraceStep)
     int mode;        // 0: z-range bounded, 1: full march
 };

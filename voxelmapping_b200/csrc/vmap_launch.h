@@ -117,7 +117,7 @@ cudaError_t launch_reset(const DevMap& m, bool whole, const Launcher& l, cudaStr
 template <class V>
 cudaError_t launch_zrange(const V& views, const Launcher& l, cudaStream_t s);
 template <class V>
-cudaError_t launch_raycast(const V& views, int fmt, const Launcher& l, cudaStream_t s);
+cudaError_t launch_raycast(const V& views, int fmt, bool wide, const Launcher& l, cudaStream_t s);  // wide: any view is
 template <class V>
 cudaError_t launch_normals(const V& views, int totalTiles, const Launcher& l, cudaStream_t s);
 cudaError_t launch_phong(const float4* vmap, size_t vpitch, const float4* nmap, size_t npitch, uchar4* rgba,
