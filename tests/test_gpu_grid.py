@@ -1,6 +1,6 @@
 """The block grid behind the ray marcher's lookups changes no result: maps of
-different capacity (grids of 32, 64 and 128 cells per axis, with and without
-two blocks in one cell) and maps far from the origin (the ray marcher's wide
+different capacity (grids of 16 to 128 cells per axis, with and without two blocks in
+one cell, and no grid) and maps far from the origin (the ray marcher's wide
 form) render, bit for bit, what a large map does; and a reset or a loaded
 snapshot leaves no stale entry."""
 import numpy as np
@@ -51,20 +51,21 @@ def same(a, b):
     assert sum(int(np.isfinite(x).sum()) for x in a) > 1000
 
 
-# shift in metres: at 16 mm the narrow range ends at 2,081 m (32 cells), 4,178 m (64) and 8,372 m (128)
+# shift in metres: at 16 mm the narrow range ends at 1,032 m (2^12 blocks, 16 cells on the shortest axis), 2,080 m
+# (2^15, 32) and 4,178 m (2^18, 64)
 @pytest.mark.parametrize("shift", [0.0, -900.0, 1500.0, 3000.0, -5000.0])
 @pytest.mark.parametrize("mode", [0, 1])
 def test_capacities_agree(shift, mode):
     fs = frames(2, np.array([shift, -0.5 * shift, 0.25 * shift]))
     poses = [fs[1][1], fs[0][1]]
-    want = drive(new_map(1 << 16, mode=mode), fs, poses)
+    want = drive(new_map(1 << 18, mode=mode), fs, poses)
     for blocks in (1 << 12, 1 << 15):
         same(drive(new_map(blocks, mode=mode), fs, poses), want)
 
 
 @pytest.mark.parametrize("fmt", ["ref", "f16", "i16"])
 def test_formats_and_shared_cells(fmt):
-    """4 mm voxels: the room spans 125 blocks, so cells of the 64-cell grid are shared."""
+    """4 mm voxels: the room spans 125 blocks, more than the smaller grid's 64 x 32 x 32 cells."""
     fs = [(d, p) for d, p in frames(1, np.zeros(3))]
     poses = [fs[0][1]]
     want = drive(new_map(1 << 18, fmt, vs=0.004), fs, poses)
@@ -104,3 +105,22 @@ def test_batch_with_a_far_map_takes_the_wide_form():
     drive(m, [near[0]] + [near[1]] * 3, [])
     w = torch.empty((H, W, 4), device="cuda")
     same([v[0].cpu().numpy(), n[0].cpu().numpy()], [m.RenderScene(None, near[1][1], w).cpu().numpy(), w.cpu().numpy()])
+
+
+def test_tiny_map_without_a_grid():
+    import torch
+    d = torch.zeros((H, W), dtype=torch.int16, device="cuda")
+    d[60:66, 80:86] = 1000
+    out = []
+    for blocks in (8, 1 << 12):
+        vm = VoxelMapping(W, H, K, voxel_format="f32", with_color=False)
+        vm.CreateMap(0, blocks, 0.016)
+        for _ in range(3):
+            vm.FuseDepth(d, np.eye(4))
+        p = np.eye(4)
+        p[0, 3] = 0.01
+        out.append([vm.RenderScene(None, x).cpu().numpy() for x in (np.eye(4), p)])
+        st = vm.stats()
+        assert st["error_flags"] == 0 and 0 < st["allocated_blocks"] <= 8
+    assert np.isfinite(out[0][0]).any()
+    assert all(np.array_equal(a, b, equal_nan=True) for a, b in zip(*out))

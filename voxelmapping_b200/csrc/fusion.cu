@@ -121,18 +121,8 @@ __global__ void __launch_bounds__(256, 6) fuse_kernel(V views)
 __global__ void __launch_bounds__(256) reset_kernel(DevMap m, bool whole)
 {
     const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x, nt = (size_t)gridDim.x * blockDim.x;
-    const size_t slots = (size_t)m.nBucket * kSlots;
-    for (size_t i = t; i < slots; i += nt) m.slots[i] = make_ulonglong2(kEmptyKey, ~0ull);
     const bool unknown = whole || m.ctr[C_UNKNOWN];
-    if (unknown) {
-        const size_t cells = grid_cells(m.capacity);
-        for (size_t i = t; i < cells; i += nt) m.grid[i] = 0ull;
-        for (size_t i = t; i < cells / 64; i += nt) m.occ[i] = 0ull;
-        for (size_t i = t; i < cells / 4096; i += nt) m.occ2[i] = 0ull;
-    } else {
-        const int n = allocated_blocks(m);
-        for (size_t i = t; i < (size_t)n; i += nt) grid_clear(m, m.blockKeys[i]);
-    }
+    index_clear(m, unknown, unknown ? 0 : allocated_blocks(m), t, nt);
     if (whole) return;  // the host clears the pool
     // block bytes are a multiple of 16 in every format, and the pool is 256-byte aligned
     const size_t blocks = unknown ? (size_t)m.capacity : (size_t)allocated_blocks(m);

@@ -142,7 +142,7 @@ void make_view(const vmap_map* m, const double pose[16], MapView& v)
     v.out.rts = m->cfg.truncation / m->cfg.voxel_size;
     if (pose) {
         const double reach = view_reach(m, pose);
-        v.out.wide = !(reach < narrow_limit(m->dm.gridLog2));
+        v.out.wide = !m->dm.grid || !(reach < narrow_limit(m->dm.g));
         // a jump rounds a position by half a unit in the last place, 2^-24 of
         // it; a cube is crossed in some 50 jumps at most
         v.out.slack = (float)(0.05 + reach * 0x1p-17);
@@ -373,30 +373,38 @@ vmap_status resolve_config(const vmap_config* cfg_in, vmap_config& cfg)
     return VMAP_OK;
 }
 
-// Device buffers of a map, in order, each starting on a 256-byte boundary:
-// hash slots, block keys, voxel pool, counters, visible list, z-range tiles
-// (min, max), triangle count, neighbour links, block grid (bricks,
-// regions, cells).
+// Device buffers of a map, each starting on a 256-byte boundary: hash table and
+// neighbour links with the block grid behind them (INDEX), block keys, voxel
+// pool, counters, visible list, z-range tiles (min, max), triangle count. The
+// index takes the bytes of 16-byte hash entries and 7 links per block; its
+// entries are 12 bytes, its links 6, and the grid fills what is left.
 struct MapLayout {
-    enum { SLOTS, KEYS, POOL, CTR, VIS, ZMIN, ZMAX, NTRI, NBR, OCC, OCC2, GRID, N };
+    enum { INDEX, KEYS, POOL, CTR, VIS, ZMIN, ZMAX, NTRI, N };
     size_t off[N + 1];
+    size_t hkeys, hslots, nbr, grid;  // offsets within INDEX
+    int gridLog2;                     // 2^gridLog2 cells, 0: no grid
 };
 
 MapLayout map_layout(const vmap_config& cfg)
 {
     const size_t nslots = (size_t)cfg.num_buckets * kSlots, cap = (size_t)cfg.num_blocks;
     const size_t ntiles = (size_t)((cfg.width + kZTile - 1) / kZTile) * ((cfg.height + kZTile - 1) / kZTile);
-    const size_t sz[MapLayout::N] = {nslots * sizeof(ulonglong2), cap * sizeof(unsigned long long),
+    auto up = [](size_t n) { return (n + 255) / 256 * 256; };
+    const size_t index = up(nslots * 16) + up(cap * 7 * sizeof(int));
+    const size_t sz[MapLayout::N] = {index, cap * sizeof(unsigned long long),
                                      cap * vmap_block_bytes(cfg.voxel_format, cfg.with_color),
                                      C_COUNT * sizeof(unsigned), cap * sizeof(int),
                                      ntiles * sizeof(unsigned long long), ntiles * sizeof(unsigned long long),
-                                     sizeof(unsigned), cap * 7 * sizeof(int),
-                                     grid_cells(cfg.num_blocks) / 64 * sizeof(unsigned long long),
-                                     grid_cells(cfg.num_blocks) / 4096 * sizeof(unsigned long long),
-                                     grid_cells(cfg.num_blocks) * sizeof(unsigned long long)};
+                                     sizeof(unsigned)};
     MapLayout l;
     l.off[0] = 0;
-    for (int i = 0; i < MapLayout::N; ++i) l.off[i + 1] = (l.off[i] + sz[i] + 255) / 256 * 256;
+    for (int i = 0; i < MapLayout::N; ++i) l.off[i + 1] = up(l.off[i] + sz[i]);
+    l.hkeys = 0;
+    l.hslots = nslots * sizeof(unsigned long long);
+    l.nbr = l.hslots + nslots * sizeof(int);
+    l.grid = (l.nbr + cap * 6 * sizeof(int) + 7) / 8 * 8;
+    l.gridLog2 = 0;
+    for (int k = 6; k <= 24 && l.grid + grid_words(k) * sizeof(unsigned long long) <= index; ++k) l.gridLog2 = k;
     return l;
 }
 
@@ -431,10 +439,6 @@ vmap_status build_map(const vmap_config& cfg, unsigned char* base, cudaStream_t 
     const size_t blockBytes = vmap_block_bytes(cfg.voxel_format, cfg.with_color);
     m->poolBytes = (size_t)cfg.num_blocks * blockBytes;
     const MapLayout l = map_layout(cfg);
-    void** ptrs[MapLayout::N] = {(void**)&m->dm.slots, (void**)&m->dm.blockKeys, (void**)&m->dm.pool,
-                                 (void**)&m->dm.ctr, (void**)&m->dm.visList, (void**)&m->zmin, (void**)&m->zmax,
-                                 (void**)&m->dNtri, (void**)&m->dm.nbr, (void**)&m->dm.occ, (void**)&m->dm.occ2,
-                                 (void**)&m->dm.grid};
     if (base) {
         m->deviceBytes = l.off[MapLayout::N];
     } else {
@@ -446,7 +450,23 @@ vmap_status build_map(const vmap_config& cfg, unsigned char* base, cudaStream_t 
         }
         base = m->arena;
     }
-    for (int i = 0; i < MapLayout::N; ++i) *ptrs[i] = base + l.off[i];
+    unsigned char* index = base + l.off[MapLayout::INDEX];
+    m->dm.keys = reinterpret_cast<unsigned long long*>(index + l.hkeys);
+    m->dm.slots = reinterpret_cast<int*>(index + l.hslots);
+    m->dm.nbr = reinterpret_cast<int*>(index + l.nbr);
+    if (l.gridLog2) {
+        m->dm.g = grid_shape(l.gridLog2);
+        m->dm.occ2 = reinterpret_cast<unsigned long long*>(index + l.grid);
+        m->dm.occ = m->dm.occ2 + (grid_words(l.gridLog2) - ((size_t)1 << l.gridLog2) - ((size_t)1 << (l.gridLog2 - 6)));
+        m->dm.grid = m->dm.occ + ((size_t)1 << (l.gridLog2 - 6));
+    }
+    m->dm.blockKeys = reinterpret_cast<unsigned long long*>(base + l.off[MapLayout::KEYS]);
+    m->dm.pool = base + l.off[MapLayout::POOL];
+    m->dm.ctr = reinterpret_cast<unsigned*>(base + l.off[MapLayout::CTR]);
+    m->dm.visList = reinterpret_cast<int*>(base + l.off[MapLayout::VIS]);
+    m->zmin = reinterpret_cast<unsigned long long*>(base + l.off[MapLayout::ZMIN]);
+    m->zmax = reinterpret_cast<unsigned long long*>(base + l.off[MapLayout::ZMAX]);
+    m->dNtri = reinterpret_cast<unsigned*>(base + l.off[MapLayout::NTRI]);
     if ((e = cudaHostAlloc((void**)&m->hCtr, C_COUNT * sizeof(unsigned), cudaHostAllocDefault)) != cudaSuccess) {
         vmap_status st = cuda_fail(e, "cudaHostAlloc");
         free_all(m);
@@ -456,7 +476,6 @@ vmap_status build_map(const vmap_config& cfg, unsigned char* base, cudaStream_t 
     m->dm.nBucket = cfg.num_buckets;
     m->dm.bucketMagic = bucket_magic((unsigned)cfg.num_buckets);
     m->dm.capacity = cfg.num_blocks;
-    m->dm.gridLog2 = grid_log2(cfg.num_blocks);
     m->dm.blockBytes = (int)blockBytes;
     m->dm.vs = cfg.voxel_size;
     m->dm.mu = cfg.truncation;

@@ -76,21 +76,26 @@ struct March {
         return 1.f;
     }
 
-    // Grid entry of the block of floor codes (ix, iy, iz), and the slot it
-    // gives (-1: absent). Narrow codes are not the coordinates, but agree with
-    // them in the bits that the cell and the tag use.
-    static __device__ __forceinline__ unsigned long long entry(const DevMap& m, int ix, int iy, int iz)
+    // Block coordinates of a floor code. Narrow codes themselves agree with
+    // the coordinates in the bits that the grid's cells and tags use.
+    static __device__ __forceinline__ int block(int i)
     {
-        const int bx = ix >> 3, by = iy >> 3, bz = iz >> 3;
-        return ld_map<NC>(m.grid + ((size_t)grid_brick(m, bx, by, bz) * 64 + grid_bit(bx, by, bz)));
+        if constexpr (WIDE) return i >> 3;
+        else return (i >> 3) - (__builtin_bit_cast(int, kFloorAdd) >> 3);
     }
+    // Slot that grid entry e gives the block of floor codes (ix, iy, iz), -1: absent.
     static __device__ __forceinline__ int slot_of(const DevMap& m, unsigned long long e, int ix, int iy, int iz)
     {
         const int bx = ix >> 3, by = iy >> 3, bz = iz >> 3;
         const unsigned hi = (unsigned)(e >> 32), tag = WIDE ? grid_tag(m, bx, by, bz) : grid_tag_bits(m, bx, by, bz);
         if ((!WIDE || tag) && (hi & ~kGridShared) == tag) return (int)(unsigned)e;
-        constexpr int k = WIDE ? 0 : __builtin_bit_cast(int, kFloorAdd) >> 3;
-        return hi & kGridShared ? hash_find<NC>(m, bx - k, by - k, bz - k) : -1;
+        return hi & kGridShared ? hash_find<NC>(m, block(ix), block(iy), block(iz)) : -1;
+    }
+    // Slot of the block of floor codes (ix, iy, iz).
+    static __device__ __forceinline__ int find(const DevMap& m, int ix, int iy, int iz)
+    {
+        if (WIDE && !m.grid) return hash_find<NC>(m, ix >> 3, iy >> 3, iz >> 3);
+        return slot_of(m, ld_map<NC>(grid_cell(m, grid_brick8(m, ix, iy, iz), grid_bit8(ix, iy, iz))), ix, iy, iz);
     }
 
     // read_sdf_interped (ray_tracing.cu:288-321): corners floor(p + {0,1}^3),
@@ -140,7 +145,7 @@ struct March {
     // wait for it.
     static __device__ __forceinline__ int far_slot(const DevMap& m, int slot, int cross)
     {
-        return cross == 1 || cross == 2 || cross == 4 ? ld_map<NC>(m.nbr + (7 * (size_t)slot + cross - 1)) : slot;
+        return cross == 1 || cross == 2 || cross == 4 ? ld_map<NC>(m.nbr + (6 * (size_t)slot + cross - 1)) : slot;
     }
 
     // Values of the 8 corners of c, all observed or not, from corner 0's block
@@ -183,12 +188,15 @@ struct March {
                 ok = false;
             }
         } else {  // several axes: independent links, then independent corners
-            const int* L = m.nbr + 7 * (size_t)slot;
+            const int* L = m.nbr + 6 * (size_t)slot;
 #pragma unroll
             for (int k = 1; k < 8; ++k) {
                 const int vx = (k & 1) ? c.x1 : c.x0, vy = (k & 2) ? c.y1 : c.y0, vz = (k & 4) ? c.z1 : c.z0;
                 const int o = k & cross;  // corner k's block, as an offset from corner 0's
-                s[k] = voxel(m, o ? ld_map<NC>(L + o - 1) : slot, vx, vy, vz, v);
+                int at_slot = slot;
+                if (k == 7 && o == 7) at_slot = find(m, vx, vy, vz);  // no link to the far one on all axes
+                else if (o) at_slot = ld_map<NC>(L + o - 1);
+                s[k] = voxel(m, at_slot, vx, vy, vz, v);
                 ok &= v;
             }
         }
@@ -298,17 +306,20 @@ struct March {
     // three reads do not depend on one another.
     static __device__ __forceinline__ void settle(const DevMap& m, Ray& r, int ix, int iy, int iz, bool same_brick)
     {
-        const int bx = ix >> 3, by = iy >> 3, bz = iz >> 3;
-        const int bit = grid_bit(bx, by, bz);
-        const int brick = grid_brick(m, bx, by, bz);
-        const unsigned long long* cell = m.grid + ((size_t)brick * 64 + bit);
+        if (WIDE && !m.grid) {
+            r.cmask = 7;
+            r.cblk = hash_find<NC>(m, ix >> 3, iy >> 3, iz >> 3);
+            return;
+        }
+        const int brick8 = grid_brick8(m, ix, iy, iz), bit8 = grid_bit8(ix, iy, iz);
+        const unsigned long long* cell = grid_cell(m, brick8, bit8);
         unsigned long long e = 0ull;
         r.cmask = 7;
         if (same_brick) {
-            if ((r.bits >> bit) & 1ull) e = ld_map<NC>(cell);
+            if ((r.bits >> (bit8 >> 3)) & 1ull) e = ld_map<NC>(cell);
         } else {
-            const unsigned long long above = ld_map<NC>(m.occ2 + grid_region(m, bx, by, bz));
-            r.bits = ld_map<NC>(m.occ + brick);
+            const unsigned long long above = ld_map<NC>(m.occ2 + grid_region(m, ix, iy, iz));
+            r.bits = ld_map<NC>(grid_occ(m, brick8));
             e = ld_map<NC>(cell);
             if (r.bits == 0ull) r.cmask = above == 0ull ? 127 : 31;
         }
@@ -452,7 +463,7 @@ struct March {
             r.res = fma3(__fmul_rn(r.sdf, o.rts), r.dir, r.res);
             const int ix = fl(r.res.x), iy = fl(r.res.y), iz = fl(r.res.z);
             int slot = r.cblk;
-            if (moved(r, ix, iy, iz) & ~7) slot = slot_of(v.m, entry(v.m, ix, iy, iz), ix, iy, iz);
+            if (moved(r, ix, iy, iz) & ~7) slot = find(v.m, ix, iy, iz);
             bool valid = false;
             const Corners c = corners(r.res, ix, iy, iz);
             const int cross = c.cross();
@@ -465,7 +476,7 @@ struct March {
                 for (int k = 0; k < 8; ++k) {
                     const int vx = (k & 1) ? c.x1 : c.x0, vy = (k & 2) ? c.y1 : c.y0, vz = (k & 4) ? c.z1 : c.z0;
                     bool ok;
-                    e[k] = k & cross ? voxel(v.m, slot_of(v.m, entry(v.m, vx, vy, vz), vx, vy, vz), vx, vy, vz, ok) : 1.f;
+                    e[k] = k & cross ? voxel(v.m, find(v.m, vx, vy, vz), vx, vy, vz, ok) : 1.f;
                 }
             }
             const float s = lerp8(e, c.ax, c.ay, c.az);

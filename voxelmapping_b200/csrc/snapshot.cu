@@ -55,13 +55,13 @@ __device__ void hash_insert_slot(const DevMap& m, unsigned long long key, unsign
     int b = ref_hash_fast(c.x, c.y, c.z, m.nBucket, m.bucketMagic);
 #pragma unroll 1
     for (int p = 0; p < kMaxProbe; ++p) {
-        ulonglong2* s = m.slots + (size_t)b * kSlots;
+        unsigned long long* s = m.keys + (size_t)b * kSlots;
 #pragma unroll 1
         for (int i = 0; i < kSlots; ++i) {
-            unsigned long long cur = __ldcg(&s[i].x);
-            if (cur == kEmptyKey) cur = atomicCAS(&s[i].x, kEmptyKey, key);
+            unsigned long long cur = __ldcg(s + i);
+            if (cur == kEmptyKey) cur = atomicCAS(s + i, kEmptyKey, key);
             if (cur == kEmptyKey) {
-                s[i].y = (unsigned long long)slot;
+                m.slots[(size_t)b * kSlots + i] = (int)slot;
                 grid_insert(m, c.x, c.y, c.z, slot);
                 return;
             }
@@ -91,17 +91,9 @@ __global__ void rebuild_hash_kernel(DevMap m, unsigned n, unsigned flags)
     }
 }
 
-__global__ void clear_slots_kernel(DevMap m)
+__global__ void clear_index_kernel(DevMap m)
 {
-    const size_t n = (size_t)m.nBucket * kSlots;
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
-        m.slots[i] = make_ulonglong2(kEmptyKey, ~0ull);
-    const size_t cells = grid_cells(m.capacity);
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < cells; i += (size_t)gridDim.x * blockDim.x) {
-        m.grid[i] = 0ull;
-        if (i < cells / 64) m.occ[i] = 0ull;
-        if (i < cells / 4096) m.occ2[i] = 0ull;
-    }
+    index_clear(m, true, 0, (size_t)blockIdx.x * blockDim.x + threadIdx.x, (size_t)gridDim.x * blockDim.x);
 }
 
 int sm_count()
@@ -207,7 +199,7 @@ vmap_status vmap_snapshot_load(vmap_map* map, const void* src, uint64_t bytes, v
     if (st.allocated_blocks > n)
         SNAP_CK(cudaMemsetAsync(m.pool + (size_t)n * m.blockBytes, 0, (size_t)(st.allocated_blocks - n) * m.blockBytes, s));
     SNAP_CK(cudaMemsetAsync(m.ctr, 0, C_UNKNOWN * sizeof(unsigned), s));
-    clear_slots_kernel<<<grid_for((size_t)m.nBucket * kSlots + grid_cells(m.capacity)), 256, 0, s>>>(m);
+    clear_index_kernel<<<grid_for((size_t)m.nBucket * kSlots), 256, 0, s>>>(m);
     SNAP_CK(cudaGetLastError());
     if (n) {
         SNAP_CK(cudaMemcpyAsync(m.blockKeys, p + h.keys_offset, 8ull * n, cudaMemcpyDefault, s));

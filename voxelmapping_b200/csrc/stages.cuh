@@ -267,29 +267,31 @@ __device__ __forceinline__ void fuse_voxels(const MapView& v, int slot, int v0)
 
 // ------------------------------------------------------------------ z-range
 // Neighbour links of the blocks allocated since the last render,
-// [ctr[C_LINKED], allocated): each new block is 14 independent tasks, one
-// lookup each - its 7 forward links, and the link of each of its 7 backward
+// [ctr[C_LINKED], allocated): each new block is 12 independent tasks, one
+// lookup each - its 6 forward links, and the link of each of its 6 backward
 // neighbours that points at it. Two new neighbours write each other's link
 // with the same value, so the order of the writes does not matter.
+constexpr int kLinkTasks = 12;
+
 __device__ __forceinline__ int links_pending(const MapView& v)
 {
     if (!v.out.vmap) return 0;
     const int done = (int)*((volatile const unsigned*)(v.m.ctr + C_LINKED));
     const int n = allocated_blocks(v.m);
-    return n > done ? 14 * (n - done) : 0;
+    return n > done ? kLinkTasks * (n - done) : 0;
 }
 
 template <bool NC>
 __device__ __forceinline__ void link_task(const DevMap& m, int t)
 {
-    const int slot = (int)*((volatile const unsigned*)(m.ctr + C_LINKED)) + t / 14;
-    const int k = 1 + (t % 14) / 2, dx = k & 1, dy = (k >> 1) & 1, dz = (k >> 2) & 1;
+    const int slot = (int)*((volatile const unsigned*)(m.ctr + C_LINKED)) + t / kLinkTasks;
+    const int k = 1 + (t % kLinkTasks) / 2, dx = k & 1, dy = (k >> 1) & 1, dz = (k >> 2) & 1;
     const int3 b = unpack_key(m.blockKeys[slot]);
     if (t & 1) {  // a backward neighbour's link to this block
         const int e = block_find<NC>(m, b.x - dx, b.y - dy, b.z - dz);
-        if (e >= 0) m.nbr[7 * (size_t)e + k - 1] = slot;
+        if (e >= 0) m.nbr[6 * (size_t)e + k - 1] = slot;
     } else {
-        m.nbr[7 * (size_t)slot + k - 1] = block_find<NC>(m, b.x + dx, b.y + dy, b.z + dz);
+        m.nbr[6 * (size_t)slot + k - 1] = block_find<NC>(m, b.x + dx, b.y + dy, b.z + dz);
     }
 }
 

@@ -50,23 +50,33 @@ struct Xf {
     float m[3][4];
 };
 
+// Shape of a map's block grid: log2 of the cells per axis; the bits of a voxel
+// coordinate that number its brick, and the bytes per brick along y and z as
+// multiples of them; the bits of a region number and its strides.
+struct GridShape {
+    int lx, ly, lz;
+    int bx, by, bz, sy, sz;
+    int rx, ry, rz, ry_shift, rz_shift;
+};
+
 struct DevMap {
-    ulonglong2* slots;             // nBucket * kSlots: {packed block coordinates, pool slot or -1}
+    unsigned long long* keys;      // hash table, nBucket * kSlots: packed block coordinates
+    int* slots;                    // pool slot of each hash entry, or -1
     unsigned long long* blockKeys; // capacity: key of each allocated block
     unsigned char* pool;           // capacity * blockBytes
     unsigned* ctr;                 // C_COUNT counters
     int* visList;                  // capacity: visible block slots
-    // forward neighbour links: nbr[7 * s + k - 1] = pool slot of the block at
-    // (bx + (k & 1), by + (k >> 1 & 1), bz + (k >> 2 & 1)) for block slot s,
-    // or -1 while that block is not allocated; set for the blocks below
-    // ctr[C_LINKED] (all of them once a z-range pass has run)
-    int* nbr;                      // capacity * 7
-    // block grid: a torus of 2^gridLog2 cells per axis over the block
-    // coordinates, in bricks of 4 x 4 x 4 cells (grid_cell)
+    // forward neighbour links: nbr[6 * s + k - 1] = pool slot of the block at
+    // (bx + (k & 1), by + (k >> 1 & 1), bz + (k >> 2 & 1)) for block slot s and
+    // k = 1 .. 6, or -1 while that block is not allocated; set for the blocks
+    // below ctr[C_LINKED] (all of them once a z-range pass has run)
+    int* nbr;                      // capacity * 6
+    // block grid: a torus of 2^log2[a] cells on axis a over the block
+    // coordinates, in bricks of 4 x 4 x 4 cells
     unsigned long long* occ;       // one word per brick: bit set when a block was allocated in that cell
-    unsigned long long* occ2;      // one word per 4 x 4 x 4 bricks: bit set when the brick's word is not zero
-    unsigned long long* grid;      // one entry per cell (grid_entry)
-    int gridLog2;
+    unsigned long long* occ2;      // one word per 4 x 4 x 4 bricks: zero when all their words are
+    unsigned long long* grid;      // one entry per cell; NULL: the map has no grid
+    GridShape g;
     unsigned long long bucketMagic;  // ceil(2^64 / nBucket): remainder by multiplication
     int nBucket;
     int capacity;
@@ -158,50 +168,74 @@ __device__ __forceinline__ int local_idx(int vx, int vy, int vz)
 // brick answers for 64 blocks at once, that of a region for 64 bricks: a ray
 // crosses empty space with a look at the words per empty cube (up to 16 blocks
 // wide) instead of one per block.
-// 8 cells per block of a large pool's surface share would be wasted on small
-// ones, so the side follows the capacity: 32 up to 2^12 blocks (0.26 MB), 64
-// up to 2^15 (2.1 MB), 128 above (17 MB; a 4 m room at 5 mm spans 100 blocks).
+// The grid lives in the bytes that a map's hash table and links would take with
+// 16-byte entries and a seventh link, about 2 cells per block of the default
+// bucket count: 128 x 128 x 128 at 2^20 blocks, 64 x 64 x 32 at 2^16. A map with
+// few buckets may have none; its lookups go to the hash table.
 constexpr unsigned kGridValid = 1u << 30, kGridShared = 1u << 31;  // in an entry's high word
 
-__host__ __device__ constexpr int grid_log2(int capacity)
+// bytes of a grid of 2^k cells: entries, brick words, region words
+__host__ __device__ constexpr size_t grid_words(int k)
 {
-    return capacity <= (1 << 12) ? 5 : capacity <= (1 << 15) ? 6 : 7;
+    return ((size_t)1 << k) + ((size_t)1 << (k - 6)) + (k > 15 ? (size_t)1 << (k - 12) : 8);
+}
+
+__host__ inline GridShape grid_shape(int k)
+{
+    GridShape g;
+    g.lx = (k + 2) / 3;
+    g.ly = (k - g.lx + 1) / 2;
+    g.lz = k - g.lx - g.ly;
+    auto regions = [](int l) { return l > 4 ? l - 4 : 0; };
+    g.bx = ((1 << (g.lx - 2)) - 1) << 5;
+    g.by = ((1 << (g.ly - 2)) - 1) << 5;
+    g.bz = ((1 << (g.lz - 2)) - 1) << 5;
+    g.sy = 1 << (g.lx + 2);
+    g.sz = 1 << (g.lx + g.ly);
+    g.rx = (1 << regions(g.lx)) - 1;
+    g.ry = (1 << regions(g.ly)) - 1;
+    g.rz = (1 << regions(g.lz)) - 1;
+    g.ry_shift = regions(g.lx);
+    g.rz_shift = regions(g.lx) + regions(g.ly);
+    return g;
 }
 
 // Voxel coordinates below which every block is within the tag's range and every
 // floor within 2^22, with room for a ray's last steps.
-__host__ __device__ constexpr double narrow_limit(int gridLog2) { return (4096 << gridLog2) - 1024; }
+__host__ inline double narrow_limit(const GridShape& g) { return (4096 << (g.lz < g.ly ? g.lz : g.ly)) - 1024; }
 
-__host__ __device__ constexpr size_t grid_cells(int capacity) { return (size_t)1 << (3 * grid_log2(capacity)); }
-
-// brick of block (x, y, z), region of 4 x 4 x 4 bricks, and the block's bit
-// within its brick (with x / 4, y / 4, z / 4: the brick's bit within its region)
-__device__ __forceinline__ int grid_brick(const DevMap& m, int x, int y, int z)
+// Of the block of voxel (x, y, z): byte offset of its brick's 64 entries, of its
+// entry among them (8 times its bit in the brick's occupancy word), and its
+// region of 4 x 4 x 4 bricks. Multiply-adds rather than shifts and ORs: the
+// ray marcher is short of the pipe that does those.
+__device__ __forceinline__ int grid_brick8(const DevMap& m, int x, int y, int z)
 {
-    const int l = m.gridLog2 - 2, mask = (1 << l) - 1;
-    return ((((z >> 2) & mask) << l | ((y >> 2) & mask)) << l) | ((x >> 2) & mask);
+    return (x & m.g.bx) * 16 + (y & m.g.by) * m.g.sy + (z & m.g.bz) * m.g.sz;
 }
+__device__ __forceinline__ int grid_bit8(int x, int y, int z) { return (x & 24) + (y & 24) * 4 + (z & 24) * 16; }
 __device__ __forceinline__ int grid_region(const DevMap& m, int x, int y, int z)
 {
-    const int l = m.gridLog2 - 4, mask = (1 << l) - 1;
-    return ((((z >> 4) & mask) << l | ((y >> 4) & mask)) << l) | ((x >> 4) & mask);
+    return ((z >> 7) & m.g.rz) << m.g.rz_shift | ((y >> 7) & m.g.ry) << m.g.ry_shift | ((x >> 7) & m.g.rx);
 }
-__device__ __forceinline__ int grid_bit(int x, int y, int z) { return ((z & 3) << 4) | ((y & 3) << 2) | (x & 3); }
+__device__ __forceinline__ unsigned long long* grid_cell(const DevMap& m, int brick8, int bit8)
+{
+    return reinterpret_cast<unsigned long long*>(reinterpret_cast<char*>(m.grid) + (unsigned)(brick8 + bit8));
+}
+__device__ __forceinline__ unsigned long long* grid_occ(const DevMap& m, int brick8) { return m.occ + (brick8 >> 9); }
 
 // high word of block (x, y, z)'s entry: for blocks within the tag's range, from
 // the low bits of the coordinates alone
 __device__ __forceinline__ unsigned grid_tag_bits(const DevMap& m, int x, int y, int z)
 {
-    const int l = m.gridLog2;
-    return kGridValid | ((unsigned)(x >> l) & 1023u) << 20 | ((unsigned)(y >> l) & 1023u) << 10 | ((unsigned)(z >> l) & 1023u);
+    return kGridValid | ((unsigned)(x >> m.g.lx) & 1023u) << 20 | ((unsigned)(y >> m.g.ly) & 1023u) << 10 |
+           ((unsigned)(z >> m.g.lz) & 1023u);
 }
 
 // the same for any block, 0 when its coordinates exceed the tag
 __device__ __forceinline__ unsigned grid_tag(const DevMap& m, int x, int y, int z)
 {
-    const int l = m.gridLog2;
-    const unsigned lim = 512u << l;
-    if ((unsigned)x + lim >= 2 * lim || (unsigned)y + lim >= 2 * lim || (unsigned)z + lim >= 2 * lim) return 0u;
+    const int tx = x >> m.g.lx, ty = y >> m.g.ly, tz = z >> m.g.lz;
+    if ((unsigned)(tx + 512) >= 1024u || (unsigned)(ty + 512) >= 1024u || (unsigned)(tz + 512) >= 1024u) return 0u;
     return grid_tag_bits(m, x, y, z);
 }
 
@@ -305,8 +339,8 @@ __device__ __forceinline__ T ld_map(const T* p)
 
 // ------------------------------------------------------------- hash table
 // Bucketed open hashing: bucket = reference hash of the block coordinates,
-// 4 slots per bucket (key and pool slot side by side: one 64-byte read per
-// probe, no second round trip for the value), linear probing into the next
+// 4 slots per bucket (the keys one 32-byte sector, the pool slots 16 bytes of
+// another array, read together: no second round trip for the value), linear probing into the next
 // bucket when all 4 are taken. Slots go EMPTY -> key exactly once, so the
 // filled slots of a bucket always form a prefix: a lookup stops at the first
 // EMPTY slot.
@@ -318,59 +352,74 @@ __device__ __forceinline__ int hash_find(const DevMap& m, int bx, int by, int bz
     int b = ref_hash_fast(bx, by, bz, m.nBucket, m.bucketMagic);
 #pragma unroll 1
     for (int p = 0; p < kMaxProbe; ++p) {
-        const ulonglong2* s = m.slots + (size_t)b * kSlots;
-        const ulonglong2 a0 = ld_map<NC>(s), a1 = ld_map<NC>(s + 1), a2 = ld_map<NC>(s + 2), a3 = ld_map<NC>(s + 3);
-        if (a0.x == key) return (int)a0.y;
-        if (a0.x == kEmptyKey) return -1;
-        if (a1.x == key) return (int)a1.y;
-        if (a1.x == kEmptyKey) return -1;
-        if (a2.x == key) return (int)a2.y;
-        if (a2.x == kEmptyKey) return -1;
-        if (a3.x == key) return (int)a3.y;
-        if (a3.x == kEmptyKey) return -1;
+        const ulonglong2* k = reinterpret_cast<const ulonglong2*>(m.keys + (size_t)b * kSlots);
+        const ulonglong2 k0 = ld_map<NC>(k), k1 = ld_map<NC>(k + 1);
+        const int4 s = ld_map<NC>(reinterpret_cast<const int4*>(m.slots + (size_t)b * kSlots));
+        if (k0.x == key) return s.x;
+        if (k0.x == kEmptyKey) return -1;
+        if (k0.y == key) return s.y;
+        if (k0.y == kEmptyKey) return -1;
+        if (k1.x == key) return s.z;
+        if (k1.x == kEmptyKey) return -1;
+        if (k1.y == key) return s.w;
+        if (k1.y == kEmptyKey) return -1;
         b = (b + 1 == m.nBucket) ? 0 : b + 1;
     }
     return -1;
-}
-
-// The block's slot through the grid (-1 when absent), given its brick and bit.
-template <bool NC>
-__device__ __forceinline__ int grid_find(const DevMap& m, int brick, int bit, int bx, int by, int bz)
-{
-    const unsigned long long e = ld_map<NC>(m.grid + ((size_t)brick * 64 + bit));
-    const unsigned hi = (unsigned)(e >> 32);
-    const unsigned tag = grid_tag(m, bx, by, bz);
-    if (tag && (hi & ~kGridShared) == tag) return (int)(unsigned)e;
-    return hi & kGridShared ? hash_find<NC>(m, bx, by, bz) : -1;
 }
 
 // hash_find's answer through the grid.
 template <bool NC = true>
 __device__ __forceinline__ int block_find(const DevMap& m, int bx, int by, int bz)
 {
-    return grid_find<NC>(m, grid_brick(m, bx, by, bz), grid_bit(bx, by, bz), bx, by, bz);
+    if (!m.grid) return hash_find<NC>(m, bx, by, bz);
+    const int x = bx * 8, y = by * 8, z = bz * 8;
+    const unsigned long long e = ld_map<NC>(grid_cell(m, grid_brick8(m, x, y, z), grid_bit8(x, y, z)));
+    const unsigned hi = (unsigned)(e >> 32);
+    const unsigned tag = grid_tag(m, bx, by, bz);
+    if (tag && (hi & ~kGridShared) == tag) return (int)(unsigned)e;
+    return hi & kGridShared ? hash_find<NC>(m, bx, by, bz) : -1;
 }
 
 // Enter an allocated block into the grid.
 __device__ __forceinline__ void grid_insert(const DevMap& m, int bx, int by, int bz, unsigned slot)
 {
-    const int brick = grid_brick(m, bx, by, bz), bit = grid_bit(bx, by, bz);
+    if (!m.grid) return;
+    const int x = bx * 8, y = by * 8, z = bz * 8;
+    const int brick8 = grid_brick8(m, x, y, z), bit8 = grid_bit8(x, y, z);
     const unsigned tag = grid_tag(m, bx, by, bz);
-    unsigned long long* cell = m.grid + ((size_t)brick * 64 + bit);
+    unsigned long long* cell = grid_cell(m, brick8, bit8);
     if (!tag || atomicCAS(cell, 0ull, (unsigned long long)tag << 32 | slot) != 0ull)
         atomicOr(cell, (unsigned long long)kGridShared << 32);
-    if (atomicOr(m.occ + brick, 1ull << bit) == 0ull)
-        atomicOr(m.occ2 + grid_region(m, bx, by, bz), 1ull << grid_bit(bx >> 2, by >> 2, bz >> 2));
+    if (atomicOr(grid_occ(m, brick8), 1ull << (bit8 >> 3)) == 0ull) atomicOr(m.occ2 + grid_region(m, x, y, z), 1ull);
 }
 
 // Empty the cells of an allocated block (of every block: an empty grid).
 __device__ __forceinline__ void grid_clear(const DevMap& m, unsigned long long key)
 {
+    if (!m.grid) return;
     const int3 b = unpack_key(key);
-    const int brick = grid_brick(m, b.x, b.y, b.z);
-    m.grid[(size_t)brick * 64 + grid_bit(b.x, b.y, b.z)] = 0ull;
-    m.occ[brick] = 0ull;
-    m.occ2[grid_region(m, b.x, b.y, b.z)] = 0ull;
+    const int x = b.x * 8, y = b.y * 8, z = b.z * 8, brick8 = grid_brick8(m, x, y, z);
+    *grid_cell(m, brick8, grid_bit8(x, y, z)) = 0ull;
+    *grid_occ(m, brick8) = 0ull;
+    m.occ2[grid_region(m, x, y, z)] = 0ull;
+}
+
+// Empty hash table and grid, by threads t, t + nt, ...; the grid's cells only
+// where `whole`, else those of the n allocated blocks.
+__device__ __forceinline__ void index_clear(const DevMap& m, bool whole, int n, size_t t, size_t nt)
+{
+    const size_t pairs = (size_t)m.nBucket * (kSlots / 2);
+    for (size_t i = t; i < pairs; i += nt) {
+        reinterpret_cast<ulonglong2*>(m.keys)[i] = make_ulonglong2(kEmptyKey, kEmptyKey);
+        reinterpret_cast<int2*>(m.slots)[i] = make_int2(-1, -1);
+    }
+    if (whole && m.grid) {
+        const size_t words = grid_words(m.g.lx + m.g.ly + m.g.lz);  // occ2, occ, grid are one piece
+        for (size_t i = t; i < words; i += nt) m.occ2[i] = 0ull;
+    } else {
+        for (size_t i = t; i < (size_t)n; i += nt) grid_clear(m, m.blockKeys[i]);
+    }
 }
 
 // Insert a block if absent (createBlock, map_struct.h:304-354, without its
@@ -383,12 +432,14 @@ __device__ __forceinline__ void hash_insert(const DevMap& m, int bx, int by, int
     int b = ref_hash_fast(bx, by, bz, m.nBucket, m.bucketMagic);
 #pragma unroll 1
     for (int p = 0; p < kMaxProbe; ++p) {
-        ulonglong2* s = m.slots + (size_t)b * kSlots;
-        const unsigned long long k[4] = {__ldcg(&s[0].x), __ldcg(&s[1].x), __ldcg(&s[2].x), __ldcg(&s[3].x)};
+        unsigned long long* s = m.keys + (size_t)b * kSlots;
+        const ulonglong2 k01 = __ldcg(reinterpret_cast<const ulonglong2*>(s));
+        const ulonglong2 k23 = __ldcg(reinterpret_cast<const ulonglong2*>(s) + 1);
+        const unsigned long long k[4] = {k01.x, k01.y, k23.x, k23.y};
 #pragma unroll
         for (int i = 0; i < kSlots; ++i) {
             unsigned long long cur = k[i];
-            if (cur == kEmptyKey) cur = atomicCAS(&s[i].x, kEmptyKey, key);
+            if (cur == kEmptyKey) cur = atomicCAS(s + i, kEmptyKey, key);
             if (cur == key) return;  // present (or inserted by another thread)
             if (cur == kEmptyKey) {  // this thread won the slot
                 cg::coalesced_group g = cg::coalesced_threads();
@@ -397,7 +448,7 @@ __device__ __forceinline__ void hash_insert(const DevMap& m, int bx, int by, int
                 const unsigned slot = g.shfl(first, 0) + g.thread_rank();
                 if (slot < (unsigned)m.capacity) {
                     m.blockKeys[slot] = key;
-                    s[i].y = (unsigned long long)slot;
+                    m.slots[(size_t)b * kSlots + i] = (int)slot;
                     grid_insert(m, bx, by, bz, slot);
                 } else {
                     atomicOr(m.ctr + C_ERR, VMAP_FLAG_POOL_FULL);
