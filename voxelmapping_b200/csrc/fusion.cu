@@ -84,6 +84,11 @@ __global__ void __launch_bounds__(256) visibility_kernel(V views)
 }
 
 // ----------------------------------------------------------------- fusion
+// Bound by instructions and, once these are done, by the bytes of the updated
+// voxels (2.4 TB/s of DRAM traffic at 22k visible blocks). Projecting with one
+// reciprocal per voxel, packed divisions and no conversion instructions took it
+// from 199 to 123 instructions per voxel: 49 -> 42.5 us at 640x480 / 5 mm and
+// 172 -> 137 us at 1280x720 / 4 mm (45k visible blocks), launch included.
 // A team of 512 / kFuseVoxels threads per visible block, kFuseVoxels voxels
 // of an x-row per thread; 256 / team blocks per CTA, grid-stride over the
 // visible blocks of all maps. 6 resident CTAs per SM (at most 40 registers)

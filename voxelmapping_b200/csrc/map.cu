@@ -111,6 +111,20 @@ static double view_reach(const vmap_map* m, const double pose[16])
     return reach;
 }
 
+// Whether no voxel's projection can overflow, and the products and remainders
+// of its divisions stay normal: voxels up to 2^23 voxel sizes from the origin
+// map to camera coordinates below 1e12, the quotients by a depth of at least
+// 1e-6 to below 1e26.
+static int tame_view(const vmap_map* m, const Xf& Ti)
+{
+    const vmap_config& c = m->cfg;
+    bool ok = c.voxel_size <= 1.f && c.fx < 1e8f && c.fy < 1e8f && std::fabs(c.cx) < 1e8f && std::fabs(c.cy) < 1e8f &&
+              c.width <= 1 << 22 && c.height <= 1 << 22 && c.truncation > 1e-5f && c.truncation < 1e5f;
+    for (int r = 0; r < 3; ++r)
+        for (int k = 0; k < 4; ++k) ok = ok && std::fabs(Ti.m[r][k]) < (k < 3 ? 1e4f : 1e11f);
+    return ok;
+}
+
 // The per-step view of a map: storage, camera, pose (FP64 inverse rounded to
 // FP32), no frame inputs and no render outputs yet.
 void make_view(const vmap_map* m, const double pose[16], MapView& v)
@@ -125,6 +139,8 @@ void make_view(const vmap_map* m, const double pose[16], MapView& v)
     v.cam.cy = m->cfg.cy;
     v.cam.ifx = (float)(1.0 / (double)m->cfg.fx);
     v.cam.ify = (float)(1.0 / (double)m->cfg.fy);
+    v.cam.fW = (float)m->cfg.width;
+    v.cam.fH = (float)m->cfg.height;
     v.in.active = 1;
     v.in.dscale = 1.f;
     if (pose) {
@@ -141,6 +157,7 @@ void make_view(const vmap_map* m, const double pose[16], MapView& v)
     v.out.vsinvRcp = 1.f / v.out.vsinv;
     v.out.rts = m->cfg.truncation / m->cfg.voxel_size;
     if (pose) {
+        v.cam.tame = tame_view(m, v.Ti);
         const double reach = view_reach(m, pose);
         v.out.wide = !m->dm.grid || !(reach < narrow_limit(m->dm.g));
         // a jump rounds a position by half a unit in the last place, 2^-24 of
@@ -479,6 +496,7 @@ vmap_status build_map(const vmap_config& cfg, unsigned char* base, cudaStream_t 
     m->dm.blockBytes = (int)blockBytes;
     m->dm.vs = cfg.voxel_size;
     m->dm.mu = cfg.truncation;
+    m->dm.muRcp = 1.f / cfg.truncation;
     m->dm.wmax = (float)cfg.max_weight;
     m->epoch = 0xFFFFFFFEu;  // the first render re-initialises the tiles
     vmap_status st = VMAP_OK;  // the memory may hold anything: clear the whole pool

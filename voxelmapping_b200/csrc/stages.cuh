@@ -17,6 +17,12 @@
 
 namespace vmapb {
 
+// Small whole numbers without the conversion unit, which runs at an eighth of
+// the multiply-add rate: a byte or a uint16 becomes the low mantissa bits of
+// 2^23, and floor(x) of 0 <= x < 2^22 the low bits of x + 2^23.
+__device__ __forceinline__ float small_to_float(unsigned n) { return __fsub_rn(__uint_as_float(0x4B000000u | n), 8388608.f); }
+__device__ __forceinline__ unsigned small_floor(float x) { return __float_as_uint(__fadd_rd(x, 8388608.f)); }  // + 0x4B000000
+
 // ---------------------------------------------------------------- frames
 // Depth and colour frames are inputs: nothing writes them while a kernel runs.
 template <int DT>
@@ -26,7 +32,7 @@ __device__ __forceinline__ float read_depth_t(const FrameIn& f, int x, int y)
     if constexpr (DT == VMAP_DEPTH_F32) {
         return __ldg(reinterpret_cast<const float*>(row) + x);
     } else {
-        return __fmul_rn(__uint2float_rn(__ldg(reinterpret_cast<const unsigned short*>(row) + x)), f.dscale);
+        return __fmul_rn(small_to_float(__ldg(reinterpret_cast<const unsigned short*>(row) + x)), f.dscale);
     }
 }
 
@@ -169,13 +175,149 @@ __device__ __forceinline__ void visibility_group(const MapView& v, int g, int la
 }
 
 // ----------------------------------------------------------------- fusion
+// Two floats side by side: Blackwell's packed multiply-adds work on both in one
+// instruction, each half rounded as the scalar one.
+struct F2 {
+    unsigned long long v;
+};
+__device__ __forceinline__ F2 f2(float a, float b)
+{
+    F2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ F2 f2(float a) { return f2(a, a); }
+__device__ __forceinline__ void f2_get(F2 x, float& a, float& b)
+{
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(x.v));
+}
+__device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c)
+{
+    F2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+    return r;
+}
+__device__ __forceinline__ F2 mul2(F2 a, F2 b)
+{
+    F2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ F2 add2(F2 a, F2 b)
+{
+    F2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+// div_exact of both halves; nb = -b
+__device__ __forceinline__ F2 div_exact2(F2 a, F2 nb, F2 y)
+{
+    F2 q = mul2(a, y);
+    q = fma2(fma2(nb, q, a), y, q);
+    return fma2(fma2(nb, q, a), y, q);
+}
+
+// 1 / b for normal b: the approximate reciprocal (within one unit in the last
+// place) and one Newton step, which rounds it correctly unless b's mantissa is
+// all ones (Markstein 1990), and to within 2^-24 (1 + 2^-23) then.
+__device__ __forceinline__ float rcp_newton(float b)
+{
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(b));
+    return __fmaf_rn(__fmaf_rn(-b, y, 1.f), y, y);
+}
+
+// Camera depth pz and pixel (pu, pv) of NV consecutive voxels, at (vx0 + x) *
+// voxel size, wy, wz (DepthFusionFunctor, depth_fusion.cu:148-196).
+//
+// The plain form, for any camera and pose: IEEE divisions and saturating
+// conversions. in[x]: whether the voxel projects into the image.
+template <int NV>
+__device__ __forceinline__ void project_any(const MapView& v, int vx0, float wy, float wz, float* pz, int* pu, int* pv,
+                                            bool* in)
+{
+#pragma unroll
+    for (int x = 0; x < NV; ++x) {
+        const float3 p = xf_apply(v.Ti, __fmul_rn(__int2float_rn(vx0 + x), v.m.vs), wy, wz);
+        // __float2int_rd(fx * p0 / p2 + cx + 0.5)
+        pu[x] = __float2int_rd(__fadd_rn(__fadd_rn(__fdiv_rn(__fmul_rn(v.cam.fx, p.x), p.z), v.cam.cx), 0.5f));
+        pv[x] = __float2int_rd(__fadd_rn(__fadd_rn(__fdiv_rn(__fmul_rn(v.cam.fy, p.y), p.z), v.cam.cy), 0.5f));
+        pz[x] = p.z;
+        in[x] = !(pu[x] < 0 || pv[x] < 0 || pu[x] > v.cam.W - 1 || pv[x] > v.cam.H - 1);
+    }
+}
+
+// The same numbers with one reciprocal for both divisions by a voxel's depth,
+// two voxels' divisions packed, and floors without conversions: for tame views
+// (CamParams::tame) and voxels that all lie on one side of the camera plane,
+// away from it (the depth is monotone along the row); false otherwise.
+template <int NV>
+__device__ __forceinline__ bool project_tame(const MapView& v, int vx0, float wy, float wz, float* pz, int* pu, int* pv,
+                                             bool* in)
+{
+    const Xf& t = v.Ti;
+    const float fx0 = __int2float_rn(vx0);
+    float wx[NV];
+#pragma unroll
+    for (int x = 0; x < NV; ++x) wx[x] = __fmul_rn(__fadd_rn(fx0, (float)x), v.m.vs);  // whole numbers below 2^24: exact
+    auto row = [&](int r, float* o) {  // xf_apply's row r
+        const float c0 = __fmul_rn(t.m[r][1], wy), c1 = __fmaf_rn(t.m[r][2], wz, t.m[r][3]);
+#pragma unroll
+        for (int x = 0; x < NV; ++x) o[x] = __fadd_rn(__fmaf_rn(t.m[r][0], wx[x], c0), c1);
+    };
+    row(2, pz);
+    if (!(fminf(fabsf(pz[0]), fabsf(pz[NV - 1])) > 1e-6f && (pz[0] > 0.f) == (pz[NV - 1] > 0.f))) return false;
+    F2 nz[NV / 2], y[NV / 2];
+#pragma unroll
+    for (int k = 0; k < NV / 2; ++k) {
+        nz[k] = f2(-pz[2 * k], -pz[2 * k + 1]);
+        y[k] = f2(rcp_newton(pz[2 * k]), rcp_newton(pz[2 * k + 1]));
+    }
+#pragma unroll
+    for (int a = 0; a < 2; ++a) {  // image columns, then rows
+        const float f = a ? v.cam.fy : v.cam.fx, c = a ? v.cam.cy : v.cam.cx, end = a ? v.cam.fH : v.cam.fW;
+        float q[NV];
+        row(a, q);
+#pragma unroll
+        for (int k = 0; k < NV / 2; ++k)
+            f2_get(div_exact2(f2(__fmul_rn(f, q[2 * k]), __fmul_rn(f, q[2 * k + 1])), nz[k], y[k]), q[2 * k], q[2 * k + 1]);
+#pragma unroll
+        for (int x = 0; x < NV; ++x) {
+            const float i = __fadd_rn(__fadd_rn(q[x], c), 0.5f);
+            in[x] = (a ? in[x] : true) && i >= 0.f && i < end;
+            (a ? pv : pu)[x] = (int)(small_floor(i) - 0x4B000000u);
+        }
+    }
+    return true;
+}
+
+// One blended colour plane of two voxels: (unsigned char)(ca o + cb n), with o
+// and n the bytes of c and of the pixels pa, pb at places `at` and plane. The
+// conversions are byte moves into and out of the low mantissa bits of 2^23
+// (the sum with 2^23 rounded down truncates); ca, cb are 0.7, 0.3, or 0, 1 for
+// a voxel seen for the first time.
+__device__ __forceinline__ unsigned blend2(unsigned c, unsigned pa, unsigned pb, int plane, int at, F2 ca, F2 cb, bool oka,
+                                           bool okb)
+{
+    auto byte = [](unsigned w, int i) { return __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7440 + i)); };
+    const F2 off = f2(-8388608.f);
+    const F2 o = add2(f2(byte(c, at), byte(c, at + 1)), off), n = add2(f2(byte(pa, plane), byte(pb, plane)), off);
+    float ra, rb;
+    f2_get(fma2(ca, o, mul2(cb, n)), ra, rb);
+    constexpr unsigned put[4] = {0x3214, 0x3240, 0x3410, 0x4210};
+    if (oka) c = __byte_perm(c, small_floor(ra), put[at]);
+    if (okb) c = __byte_perm(c, small_floor(rb), put[at + 1]);
+    return c;
+}
+
 // DepthFusionFunctor / ImageFusionFunctor for the NV (4 or 8) consecutive
 // voxels v0 .. v0 + NV - 1 of an x-row of block `slot` (one vector of NV
-// voxel words, one NV-byte word per colour plane). The projections come
-// first: each projected pixel's depth and colour are loaded right after its
-// projection, and the group's voxel words and colour planes only when one of
-// its voxels updates, so groups behind the surface or outside the frame move
-// no voxel bytes. Nothing is written unless a voxel updates.
+// voxel words, one NV-byte word per colour plane). The projections and depths
+// come first; the group's voxel words and colour planes and the pixels'
+// colours are loaded only when one of its voxels updates, so groups behind
+// the surface or outside the frame move no voxel bytes. Nothing is written
+// unless a voxel updates. A voxel's first update is the running average with
+// weight 0 of a zero TSDF, (0 * 0 + sdf) / 1.
 template <int FMT, bool COLOR, int DT, int NV = 4>
 __device__ __forceinline__ void fuse_block(const MapView& v, int slot, int v0)
 {
@@ -185,63 +327,71 @@ __device__ __forceinline__ void fuse_block(const MapView& v, int slot, int v0)
     const DevMap& m = v.m;
     const int lx0 = v0 & 7, ly = (v0 >> 3) & 7, lz = v0 >> 6;
     const int3 bp = unpack_key(m.blockKeys[slot]);
-    Word* blk = L::words_rw(m, slot);
     static_assert(NV == 4 || NV == 8, "4 or 8 voxels of an x-row");
-    Word w[NV];
-    unsigned char c[3][NV];
-    unsigned char* crow = reinterpret_cast<unsigned char*>(blk) + L::kRgbOff + v0;
     const int vx0 = bp.x * 8 + lx0;
     const float wy = __fmul_rn(__int2float_rn(bp.y * 8 + ly), m.vs);
     const float wz = __fmul_rn(__int2float_rn(bp.z * 8 + lz), m.vs);
     float sdfv[NV];
-    unsigned pix[NV];  // the projected pixel's colour, r | g << 8 | b << 16
-    unsigned mask = 0;
+    int pu[NV], pv[NV];
+    bool ok[NV];
+    {
+        float pz[NV], d[NV];
+        if (!v.cam.tame || !project_tame<NV>(v, vx0, wy, wz, pz, pu, pv, ok)) project_any<NV>(v, vx0, wy, wz, pz, pu, pv, ok);
 #pragma unroll
-    for (int x = 0; x < NV; ++x) {
-        const float3 p = xf_apply(v.Ti, __fmul_rn(__int2float_rn(vx0 + x), m.vs), wy, wz);
-        // __float2int_rd(fx * p0 / p2 + cx + 0.5)
-        const int u = __float2int_rd(__fadd_rn(__fadd_rn(__fdiv_rn(__fmul_rn(v.cam.fx, p.x), p.z), v.cam.cx), 0.5f));
-        const int vv = __float2int_rd(__fadd_rn(__fadd_rn(__fdiv_rn(__fmul_rn(v.cam.fy, p.y), p.z), v.cam.cy), 0.5f));
-        sdfv[x] = 0.f;
-        pix[x] = 0u;
-        if (u < 0 || vv < 0 || u > v.cam.W - 1 || vv > v.cam.H - 1) continue;
-        const float d = read_depth_t<DT>(v.in, u, vv);
-        if constexpr (COLOR) {
-            const uint8_t* px = v.in.rgb + (size_t)vv * v.in.rgbPitch + 3 * u;
-            pix[x] = (unsigned)__ldg(px) | ((unsigned)__ldg(px + 1) << 8) | ((unsigned)__ldg(px + 2) << 16);
+        for (int x = 0; x < NV; ++x) {
+            d[x] = 0.f;  // below the depth range
+            if (ok[x]) d[x] = read_depth_t<DT>(v.in, pu[x], pv[x]);
         }
-        if (isnan(d) || d > kMaxDepth || d < kMinDepth) continue;
-        const float sdf = __fsub_rn(d, p.z);
-        if (sdf < -m.mu) continue;
-        sdfv[x] = fminf(1.f, __fdiv_rn(sdf, m.mu));
-        mask |= 1u << x;
+#pragma unroll
+        for (int x = 0; x < NV; ++x) {
+            const float sdf = __fsub_rn(d[x], pz[x]);
+            sdfv[x] = fminf(1.f, div_exact(sdf, m.mu, m.muRcp));
+            // not isnan(d) || d > kMaxDepth || d < kMinDepth || sdf < -mu
+            ok[x] = d[x] >= kMinDepth && d[x] <= kMaxDepth && !(sdf < -m.mu);
+        }
     }
-    if (!mask) return;
+    bool any = false;
+#pragma unroll
+    for (int x = 0; x < NV; ++x) any = any || ok[x];
+    if (!any) return;
+    Word* blk = L::words_rw(m, slot);
+    unsigned char* crow = reinterpret_cast<unsigned char*>(blk) + L::kRgbOff + v0;
+    Word w[NV];
     load_vec<NV * sizeof(Word)>(blk + v0, w);
+    unsigned c[3][NV / 4], pix[NV];  // colour planes, 4 voxels to a word; the pixels' colours r | g << 8 | b << 16
     if constexpr (COLOR) {
 #pragma unroll
         for (int k = 0; k < 3; ++k) load_vec<NV>(crow + k * kBlockVoxels, c[k]);
-    }
 #pragma unroll
-    for (int x = 0; x < NV; ++x) {
-        if (!(mask & (1u << x))) continue;
-        const float ow = F::weight(w[x]);
-        if (ow == 0.f) {
-            w[x] = F::make(sdfv[x], 1.f);
-            if constexpr (COLOR) {
-#pragma unroll
-                for (int k = 0; k < 3; ++k) c[k][x] = (unsigned char)(pix[x] >> (8 * k));
-            }
-        } else {
-            const float os = F::tsdf(w[x]);
-            w[x] = F::make(__fdiv_rn(__fmaf_rn(os, ow, sdfv[x]), __fadd_rn(ow, 1.f)), fminf(__fadd_rn(ow, 1.f), m.wmax));
-            if constexpr (COLOR) {
-#pragma unroll
-                for (int k = 0; k < 3; ++k)
-                    c[k][x] = (unsigned char)__float2int_rz(__fmaf_rn(
-                        0.7f, __uint2float_rn(c[k][x]), __fmul_rn(0.3f, __uint2float_rn((pix[x] >> (8 * k)) & 0xffu))));
+        for (int x = 0; x < NV; ++x) {
+            pix[x] = 0u;
+            if (ok[x]) {
+                const uint8_t* px = v.in.rgb + (size_t)pv[x] * v.in.rgbPitch + 3 * pu[x];
+                pix[x] = (unsigned)__ldg(px) | ((unsigned)__ldg(px + 1) << 8) | ((unsigned)__ldg(px + 2) << 16);
             }
         }
+    }
+#pragma unroll
+    for (int x = 0; x < NV; x += 2) {
+        float ow[2], os[2], nw[2], s[2];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            ow[h] = F::weight(w[x + h]);
+            os[h] = ow[h] == 0.f ? 0.f : F::tsdf(w[x + h]);
+            nw[h] = __fadd_rn(ow[h], 1.f);
+        }
+        const F2 sum = fma2(f2(os[0], os[1]), f2(ow[0], ow[1]), f2(sdfv[x], sdfv[x + 1]));
+        f2_get(div_exact2(sum, f2(-nw[0], -nw[1]), f2(rcp_newton(nw[0]), rcp_newton(nw[1]))), s[0], s[1]);
+        if constexpr (COLOR) {
+            const F2 ca = f2(ow[0] == 0.f ? 0.f : 0.7f, ow[1] == 0.f ? 0.f : 0.7f);
+            const F2 cb = f2(ow[0] == 0.f ? 1.f : 0.3f, ow[1] == 0.f ? 1.f : 0.3f);
+#pragma unroll
+            for (int k = 0; k < 3; ++k)
+                c[k][x / 4] = blend2(c[k][x / 4], pix[x], pix[x + 1], k, x & 3, ca, cb, ok[x], ok[x + 1]);
+        }
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+            if (ok[x + h]) w[x + h] = F::make(s[h], fminf(nw[h], m.wmax));
     }
     store_vec<NV * sizeof(Word)>(blk + v0, w);
     if constexpr (COLOR) {

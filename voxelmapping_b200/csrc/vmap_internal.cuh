@@ -83,6 +83,7 @@ struct DevMap {
     int blockBytes;
     float vs;   // voxel size
     float mu;   // truncation distance
+    float muRcp; // 1.f / mu
     float wmax; // weight cap
 };
 
@@ -586,6 +587,8 @@ struct CamParams {
     int W, H;
     float fx, fy, cx, cy;
     float ifx, ify;  // (float)(1.0 / (double)f), as the reference's host code
+    float fW, fH;    // W, H
+    int tame;        // projections of any block overflow nothing, pixels below 2^22 (project_tame)
 };
 
 struct FrameIn {
