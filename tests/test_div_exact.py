@@ -41,7 +41,11 @@ def test_quotient_is_correctly_rounded():
 
 
 def test_every_16_bit_code():
+    """code / 32767 of the 16-bit formats: one correction rounds every code's
+    quotient correctly."""
     b = Fraction(32767)
     y = rn(1 / b)
-    for c in range(1, 32768, 7):
-        assert div_exact(Fraction(c), b, y) == rn(Fraction(c, 32767))
+    assert float(y) == float(np.float32(1.0) / np.float32(32767.0))
+    for c in range(1, 32769):
+        q = rn(c * y)
+        assert rn(rn(c - b * q) * y + q) == rn(Fraction(c, 32767)), c

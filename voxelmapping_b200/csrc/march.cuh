@@ -148,6 +148,17 @@ struct March {
         return cross == 1 || cross == 2 || cross == 4 ? ld_map<NC>(m.nbr + (6 * (size_t)slot + cross - 1)) : slot;
     }
 
+    // Whether all 8 words are observed, by their smallest weight: the weight is
+    // a word's float, or its high bits.
+    static __device__ __forceinline__ bool all_observed(Word w0, Word w1, Word w2, Word w3, Word w4, Word w5, Word w6, Word w7)
+    {
+        if constexpr (sizeof(Word) == 8) {
+            return fminf(fminf(fminf(w0.y, w1.y), fminf(w2.y, w3.y)), fminf(fminf(w4.y, w5.y), fminf(w6.y, w7.y))) > 0.f;
+        } else {
+            return min(min(min(w0, w1), min(w2, w3)), min(min(w4, w5), min(w6, w7))) >= 0x10000u;
+        }
+    }
+
     // Values of the 8 corners of c, all observed or not, from corner 0's block
     // `slot` (allocated), its far block and, for corners that leave it on
     // several axes, its forward neighbour links. w0: corner 0's word.
@@ -174,6 +185,17 @@ struct March {
             auto ld = [](const char* p) { return ld_map<NC>(reinterpret_cast<const Word*>(p)); };
             const Word w1 = ld(ax), w2 = ld(a + dy), w3 = ld(ax + dy), w4 = ld(a + dz), w5 = ld(ax + dz);
             const Word w6 = ld(a + dy + dz), w7 = ld(ax + dy + dz);
+            if (!gone && all_observed(w0, w1, w2, w3, w4, w5, w6, w7)) {  // most reads
+                s[0] = F::tsdf(w0);
+                s[1] = F::tsdf(w1);
+                s[2] = F::tsdf(w2);
+                s[3] = F::tsdf(w3);
+                s[4] = F::tsdf(w4);
+                s[5] = F::tsdf(w5);
+                s[6] = F::tsdf(w6);
+                s[7] = F::tsdf(w7);
+                return true;
+            }
             s[1] = value(w1, v); ok &= v;
             s[2] = value(w2, v); ok &= v;
             s[3] = value(w3, v); ok &= v;
@@ -229,6 +251,17 @@ struct March {
         r.dist_s = __fadd_rn(r.dist_s, k);
     }
 
+    // normalized(), with one reciprocal for its three divisions.
+    static __device__ __forceinline__ float3 direction(float3 v)
+    {
+        const float s = __fmaf_rn(v.x, v.x, __fmaf_rn(v.z, v.z, __fmul_rn(v.y, v.y)));
+        if (s > 0.f) {
+            const float n = __fsqrt_rn(s), y = rcp_newton(n);
+            v = make_float3(div_exact(v.x, n, y), div_exact(v.y, n, y), div_exact(v.z, n, y));
+        }
+        return v;
+    }
+
     // Start a ray at pixel (x, y); false when it finishes at once (tile with
     // no allocated block: written as a miss).
     static __device__ __forceinline__ bool init(const MapView& v, Ray& r, int x, int y)
@@ -256,7 +289,7 @@ struct March {
         const float dist_e = __fmul_rn(__fsqrt_rn(sqnorm(p1)), o.vsinv);
         float3 be = xf_apply(v.T, p1.x, p1.y, p1.z);
         be = make_float3(__fmul_rn(be.x, o.vsinv), __fmul_rn(be.y, o.vsinv), __fmul_rn(be.z, o.vsinv));
-        r.dir = normalized(make_float3(__fsub_rn(be.x, bs.x), __fsub_rn(be.y, bs.y), __fsub_rn(be.z, bs.z)));
+        r.dir = direction(make_float3(__fsub_rn(be.x, bs.x), __fsub_rn(be.y, bs.y), __fsub_rn(be.z, bs.z)));
         // reciprocals only bound the empty-block jump (taken with a 1e-3 margin):
         // approximate ones suffice; 1/(+-0) stays +-inf
         r.inv = make_float3(__fdividef(1.f, r.dir.x), __fdividef(1.f, r.dir.y), __fdividef(1.f, r.dir.z));

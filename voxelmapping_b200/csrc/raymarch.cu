@@ -19,8 +19,8 @@
 // which runs at half rate: at 640x480 the kernel issues 70 % of the time while
 // all its warps run) and, in scenes seen at grazing angles, the slowest tiles'
 // latency. Against a lookup per block through a warp-shared cache and the hash
-// table, event time of the launch, three rooms each: 48 -> 33 us at 160x120 /
-// 16 mm, 63 -> 43 at 320x240 / 8 mm, 96 -> 70 at 640x480 / 5 mm, 293 -> 240 at
+// table, event time of the launch, three rooms each: 48 -> 30 us at 160x120 /
+// 16 mm, 63 -> 39 at 320x240 / 8 mm, 96 -> 70 at 640x480 / 5 mm, 293 -> 241 at
 // 1280x720 / 4 mm, 320 -> 131 for an 800x600 full march (raycast_mode 1).
 //
 // Scheduling: the kernel is persistent. Each warp takes 8x4-pixel tiles from

@@ -217,16 +217,6 @@ __device__ __forceinline__ F2 div_exact2(F2 a, F2 nb, F2 y)
     return fma2(fma2(nb, q, a), y, q);
 }
 
-// 1 / b for normal b: the approximate reciprocal (within one unit in the last
-// place) and one Newton step, which rounds it correctly unless b's mantissa is
-// all ones (Markstein 1990), and to within 2^-24 (1 + 2^-23) then.
-__device__ __forceinline__ float rcp_newton(float b)
-{
-    float y;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(b));
-    return __fmaf_rn(__fmaf_rn(-b, y, 1.f), y, y);
-}
-
 // Camera depth pz and pixel (pu, pv) of NV consecutive voxels, at (vx0 + x) *
 // voxel size, wy, wz (DepthFusionFunctor, depth_fusion.cu:148-196).
 //

@@ -113,6 +113,16 @@ __device__ __forceinline__ float div_exact(float a, float b, float y)
     return __fmaf_rn(__fmaf_rn(-b, q, a), y, q);
 }
 
+// 1 / b for normal b: the approximate reciprocal (within one unit in the last
+// place) and one Newton step, which rounds it correctly unless b's mantissa is
+// all ones (Markstein 1990), and to within 2^-24 (1 + 2^-23) then.
+__device__ __forceinline__ float rcp_newton(float b)
+{
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(b));
+    return __fmaf_rn(__fmaf_rn(-b, y, 1.f), y, y);
+}
+
 // unproject (map_struct.h:189-194): ((ifx * (x - cx)) * z, (ify * (y - cy)) * z, z)
 __device__ __forceinline__ float3 unproject(int x, int y, float z, float ifx, float ify, float cx, float cy)
 {
@@ -477,11 +487,22 @@ __device__ __forceinline__ int allocated_blocks(const DevMap& m)
 template <int FMT>
 struct Fmt;
 
+// unpackFloat (map_struct.h:72-75), code / 32767.f, of the int16 in a word's low
+// half: the conversion by bits (the code plus 2^23 + 2^15 has it in its low
+// mantissa bits), the quotient from the rounded reciprocal and one correction,
+// which gives the correctly rounded one for each of the 65,536 codes.
+__device__ __forceinline__ float unpack_code(unsigned w)
+{
+    const float a = __fsub_rn(__uint_as_float((w & 0xffffu) ^ 0x4B008000u), 8421376.f);
+    const float y = 1.f / 32767.f;
+    const float q = __fmul_rn(a, y);
+    return __fmaf_rn(__fmaf_rn(-32767.f, q, a), y, q);
+}
+
 template <>
 struct Fmt<VMAP_VOXEL_REF> {  // reference Voxel: int16 x32767 tsdf, uint8 weight
     typedef unsigned Word;      // bits 0-15 tsdf code, 16-23 weight
-    // unpackFloat (map_struct.h:72-75): val / 32767.f
-    static __device__ __forceinline__ float tsdf(Word w) { return __fdiv_rn(__int2float_rn((short)(w & 0xffffu)), 32767.f); }
+    static __device__ __forceinline__ float tsdf(Word w) { return unpack_code(w); }
     static __device__ __forceinline__ float weight(Word w) { return __uint2float_rn((w >> 16) & 0xffu); }
     static __device__ __forceinline__ bool observed(Word w) { return (w >> 16) != 0u; }
     // packFloat (map_struct.h:77-80): (short)(val * 32767), truncation
@@ -515,7 +536,7 @@ struct Fmt<VMAP_VOXEL_F16> {
 template <>
 struct Fmt<VMAP_VOXEL_I16> {
     typedef unsigned Word;  // bits 0-15 int16 x32767 tsdf, 16-31 uint16 weight
-    static __device__ __forceinline__ float tsdf(Word w) { return __fdiv_rn(__int2float_rn((short)(w & 0xffffu)), 32767.f); }
+    static __device__ __forceinline__ float tsdf(Word w) { return unpack_code(w); }
     static __device__ __forceinline__ float weight(Word w) { return __uint2float_rn(w >> 16); }
     static __device__ __forceinline__ bool observed(Word w) { return (w >> 16) != 0u; }
     static __device__ __forceinline__ Word make(float t, float wt)
