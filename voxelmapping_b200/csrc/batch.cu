@@ -26,6 +26,14 @@ void make_view(const vmap_map* m, const double pose[16], MapView& v);
 cudaError_t next_epoch(vmap_map* m, cudaStream_t s, unsigned* epoch);
 }  // namespace vmapb
 
+// Which forms of the kernels a step's views need: the general ones when any of
+// them does.
+struct StepForms {
+    bool near;  // allocation: every fused view is near
+    bool wide;  // ray marcher: some rendered view is wide
+    bool operator!=(const StepForms& o) const { return near != o.near || wide != o.wide; }
+};
+
 struct vmap_batch {
     std::vector<vmap_map*> maps;
     int fmt;
@@ -40,7 +48,7 @@ struct vmap_batch {
     bool eventUsed[2];
     cudaGraphExec_t exec[2];
     cudaStream_t graphStream[2];  // stream each graph was recorded for
-    bool graphWide[2];            // ray marcher it was recorded with
+    StepForms graphForms[2];      // kernel forms it was recorded with
     int next;                // buffer of the next step
 };
 
@@ -101,16 +109,16 @@ vmap_status finish_create(vmap_batch* b, vmap_batch** out)
 
 // One step over the descriptors in dViews[buf]: the persistent launch, or
 // the six stage launches.
-cudaError_t enqueue_stages(vmap_batch* b, int buf, bool wide, cudaStream_t s)
+cudaError_t enqueue_stages(vmap_batch* b, int buf, const StepForms& f, cudaStream_t s)
 {
     ManyViews mv{b->dViews[buf], (int)b->maps.size(), b->dQueue};
     if (b->launcher.batchSchedule == 2) return launch_step(mv, b->dSched, b->fmt, b->launcher, s);
     cudaError_t e;
-    if ((e = launch_alloc(mv, b->totalAllocTiles, b->launcher, s)) != cudaSuccess) return e;
+    if ((e = launch_alloc(mv, b->totalAllocTiles, f.near, b->launcher, s)) != cudaSuccess) return e;
     if ((e = launch_visibility(mv, b->launcher, s)) != cudaSuccess) return e;
     if ((e = launch_fuse(mv, b->fmt, b->launcher, s)) != cudaSuccess) return e;
     if ((e = launch_zrange(mv, b->launcher, s)) != cudaSuccess) return e;
-    if ((e = launch_raycast(mv, b->fmt, wide, b->launcher, s)) != cudaSuccess) return e;
+    if ((e = launch_raycast(mv, b->fmt, f.wide, b->launcher, s)) != cudaSuccess) return e;
     return launch_normals(mv, b->totalNormalTiles, b->launcher, s);
 }
 
@@ -227,11 +235,11 @@ namespace {
 // Validates the step's frames and writes their descriptors into staging
 // buffer `buf` (after the copy out of it, recorded in the step before last,
 // has run).
-// *wide: whether a rendered view needs the wide ray marcher.
-vmap_status stage_frames(vmap_batch* b, const vmap_batch_frame* frames, cudaStream_t s, int buf, bool* wide)
+// *forms: the kernel forms the step's views need.
+vmap_status stage_frames(vmap_batch* b, const vmap_batch_frame* frames, cudaStream_t s, int buf, StepForms* forms)
 {
     const int n = (int)b->maps.size();
-    *wide = false;
+    *forms = StepForms{true, false};
     if (b->eventUsed[buf]) VMAP_BCK(cudaEventSynchronize(b->copied[buf]));
     for (int i = 0; i < n; ++i) {
         const vmap_batch_frame& f = frames[i];
@@ -280,7 +288,8 @@ vmap_status stage_frames(vmap_batch* b, const vmap_batch_frame* frames, cudaStre
         v.out.nmap = reinterpret_cast<float4*>(f.nmap_dev);
         v.out.npitch = np;
         if (render) VMAP_BCK(next_epoch(m, s, &v.out.epoch));
-        *wide |= render && v.out.wide;
+        forms->near &= !fuse || v.cam.near;
+        forms->wide |= render && v.out.wide;
     }
     return VMAP_OK;
 }
@@ -295,16 +304,16 @@ vmap_status vmap_batch_step(vmap_batch* b, const vmap_batch_frame* frames, void*
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
     const int n = (int)b->maps.size();
     const int buf = b->next;
-    bool wide;
-    const vmap_status st = stage_frames(b, frames, s, buf, &wide);
+    StepForms forms;
+    const vmap_status st = stage_frames(b, frames, s, buf, &forms);
     if (st != VMAP_OK) return st;
     const size_t bytes = sizeof(MapView) * (size_t)n;
     if (s == nullptr) {  // the legacy stream cannot be captured: launch directly
         VMAP_BCK(cudaMemcpyAsync(b->dViews[buf], b->hViews[buf], bytes, cudaMemcpyHostToDevice, s));
         VMAP_BCK(cudaEventRecord(b->copied[buf], s));
-        VMAP_BCK(enqueue_stages(b, buf, wide, s));
+        VMAP_BCK(enqueue_stages(b, buf, forms, s));
     } else {
-        if (b->exec[buf] && (b->graphStream[buf] != s || b->graphWide[buf] != wide)) {
+        if (b->exec[buf] && (b->graphStream[buf] != s || b->graphForms[buf] != forms)) {
             cudaGraphExecDestroy(b->exec[buf]);
             b->exec[buf] = nullptr;
         }
@@ -314,14 +323,14 @@ vmap_status vmap_batch_step(vmap_batch* b, const vmap_batch_frame* frames, void*
             cudaError_t e = cudaMemcpyAsync(b->dViews[buf], b->hViews[buf], bytes, cudaMemcpyHostToDevice, s);
             // an external record becomes a graph node the host can wait on
             if (e == cudaSuccess) e = cudaEventRecordWithFlags(b->copied[buf], s, cudaEventRecordExternal);
-            if (e == cudaSuccess) e = enqueue_stages(b, buf, wide, s);
+            if (e == cudaSuccess) e = enqueue_stages(b, buf, forms, s);
             cudaError_t e2 = cudaStreamEndCapture(s, &g);
             if (e == cudaSuccess) e = e2;
             if (e == cudaSuccess) e = cudaGraphInstantiate(&b->exec[buf], g, 0);
             if (g) cudaGraphDestroy(g);
             if (e != cudaSuccess) return fail(e, "vmap_batch_step capture");
             b->graphStream[buf] = s;
-            b->graphWide[buf] = wide;
+            b->graphForms[buf] = forms;
         }
         VMAP_BCK(cudaGraphLaunch(b->exec[buf], s));
     }
@@ -335,8 +344,8 @@ vmap_status vmap_batch_stall_probe(vmap_batch* b, const vmap_batch_frame* frames
     if (!b || !frames || stall_ms == 0 || stall_ms > 10000) return VMAP_ERR_INVALID_ARG;
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
     const int buf = b->next;
-    bool wide;
-    const vmap_status st = stage_frames(b, frames, s, buf, &wide);
+    StepForms forms;
+    const vmap_status st = stage_frames(b, frames, s, buf, &forms);
     if (st != VMAP_OK) return st;
     ManyViews mv{b->dViews[buf], (int)b->maps.size(), b->dQueue};
     VMAP_BCK(cudaMemcpyAsync(b->dViews[buf], b->hViews[buf], sizeof(MapView) * b->maps.size(),

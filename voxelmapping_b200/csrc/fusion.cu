@@ -13,50 +13,127 @@ namespace vmapb {
 
 // ---------------------------------------------------------------- allocation
 // A 256-thread CTA per 32 x kStageTileH-pixel tile, kStageTileH / 8 depth
-// pixels per thread. The
-// samples of a pixel's band are walked without touching global memory: each
-// block a pixel enters is staged in a CTA-wide shared-memory set, and once
-// the whole tile has been walked its distinct blocks (a few dozen) are
-// inserted into the hash table in parallel, one thread per block. A warp so
-// waits on one table round trip per tile instead of one per sample step, and
-// the block set is the one a per-sample insertion gives. The CTA of item 0
-// also clears the visible counters the next kernel accumulates into.
+// pixels per thread. The samples of a pixel's band are walked without touching
+// global memory: each block a pixel enters is staged in a CTA-wide
+// shared-memory set, and once the whole tile has been walked its distinct
+// blocks (a few dozen) are looked up in parallel, one thread per block, and the
+// missing ones inserted. A warp so waits on one table round trip per tile
+// instead of one per sample step, and the block set is the one a per-sample
+// insertion gives. The CTA of item 0 also clears the visible counters the next
+// kernel accumulates into.
+// Bound by instructions (940 per 32 pixels; 1,110 with the walk on conversions,
+// IEEE divisions and 64-bit keys): 19.8 -> 16.9 us at 640x480 / 5 mm, 43.6 ->
+// 36.2 us at 1280x720 / 4 mm, launch included.
 // 8 resident CTAs per SM (at most 32 registers) measured faster than the 6
 // that 38 registers allow (20.9 against 22.1 us per 640x480 frame).
-constexpr int kTileSet = 1024;  // open-addressed set of one tile's blocks (8 KB)
+constexpr int kTileSet = 1024;  // open-addressed set of one tile's blocks (8 KB), any view
+// The set of a near view's tile: 32-bit keys (band_keys) and a list of the
+// entries in use, so that neither the insertion nor the clearing visits the
+// empty ones. A key that finds no place in kNearProbes goes straight to the
+// table.
+constexpr int kNearSet = 512, kNearProbes = 16;
+
+__device__ __forceinline__ void near_insert(const DevMap& m, const BandBase& b, unsigned key)
+{
+    const int x = (int)(key & 1023u) + b.x, y = (int)(key >> 10 & 1023u) + b.y, z = (int)(key >> 20) + b.z;
+    // in steady state nearly every block is there already: one read tells
+    if (m.grid && block_find<false>(m, x, y, z) >= 0) return;
+    hash_insert(m, x, y, z);
+}
+
+// Tile `item` of the launch: its view, and this thread's column and first row.
+template <class V>
+__device__ __forceinline__ const MapView& alloc_tile(const V& views, const int* pre, int item, int& x, int& y0)
+{
+    const int mi = map_of(pre, views.count(), item);
+    const MapView& v = views[mi];
+    const int t = item - pre[mi], tx = (v.cam.W + 31) >> 5;
+    x = (t % tx) * 32 + (threadIdx.x & 31);
+    y0 = (t / tx) * kStageTileH + (threadIdx.x >> 5);
+    return v;
+}
+
+// Item prefix of the launch; block 0 clears the visible counters.
+template <class V>
+__device__ __forceinline__ int alloc_prologue(const V& views, int* pre)
+{
+    map_prefix(views, [](const MapView& v) { return alloc_tiles<kStageTileH>(v); }, pre);  // ends with __syncthreads
+    const int nmaps = views.count();
+    if (blockIdx.x == 0)
+        for (int i = threadIdx.x; i < nmaps; i += blockDim.x)
+            if (views[i].in.active) views[i].m.ctr[C_VISIBLE] = 0u;
+    return pre[nmaps];
+}
 
 template <class V>
 __global__ void __launch_bounds__(256, 8) alloc_kernel(V views)
 {
     stage_entry();
     __shared__ int pre[kMaxBatch + 1];
+    __shared__ unsigned set[kNearSet];
+    __shared__ unsigned short used[kNearSet];
+    __shared__ int nused;
+    for (int i = threadIdx.x; i < kNearSet; i += blockDim.x) set[i] = ~0u;
+    if (threadIdx.x == 0) nused = 0;
+    const int total = alloc_prologue(views, pre);
+    for (int item = blockIdx.x; item < total; item += gridDim.x) {
+        int x, y0;
+        const MapView& v = alloc_tile(views, pre, item, x, y0);
+        const BandBase base = band_base(v);
+#pragma unroll 1
+        for (int y = y0; y < y0 + kStageTileH; y += 8) {
+            const float d = x < v.cam.W && y < v.cam.H ? read_depth(v.in, x, y) : __int_as_float(0x7fffffff);
+            band_keys(v, base, x, y, d, threadIdx.x & 31, [&](unsigned key) {
+                unsigned h = (key * 0x9E3779B1u) >> (32 - ilog2(kNearSet));
+#pragma unroll 1
+                for (int p = 0; p < kNearProbes; ++p) {
+                    unsigned cur = *(volatile unsigned*)(set + h);
+                    if (cur == ~0u) {
+                        cur = atomicCAS(set + h, ~0u, key);
+                        if (cur == ~0u) {
+                            used[atomicAdd(&nused, 1)] = (unsigned short)h;
+                            return;
+                        }
+                    }
+                    if (cur == key) return;
+                    h = (h + 1) & (kNearSet - 1);
+                }
+                near_insert(v.m, base, key);
+            });
+        }
+        __syncthreads();
+        const int n = nused;
+        for (int i = threadIdx.x; i < n; i += blockDim.x) {
+            const int h = used[i];
+            near_insert(v.m, base, set[h]);
+            set[h] = ~0u;
+        }
+        __syncthreads();
+        if (threadIdx.x == 0) nused = 0;
+        __syncthreads();
+    }
+}
+
+// The same for launches with a view that is not near: 64-bit keys.
+template <class V>
+__global__ void __launch_bounds__(256, 6) far_alloc(V views)
+{
+    stage_entry();
+    __shared__ int pre[kMaxBatch + 1];
     __shared__ unsigned long long set[kTileSet];
     for (int i = threadIdx.x; i < kTileSet; i += blockDim.x) set[i] = kEmptyKey;
-    map_prefix(views, [](const MapView& v) { return alloc_tiles<kStageTileH>(v); }, pre);  // ends with __syncthreads
-    const int nmaps = views.count();
-    if (blockIdx.x == 0)
-        for (int i = threadIdx.x; i < nmaps; i += blockDim.x)
-            if (views[i].in.active) views[i].m.ctr[C_VISIBLE] = 0u;
-    const int total = pre[nmaps];
+    const int total = alloc_prologue(views, pre);
     for (int item = blockIdx.x; item < total; item += gridDim.x) {
-        const int mi = map_of(pre, nmaps, item);
-        const MapView& v = views[mi];
-        const DevMap& m = v.m;
-        const int t = item - pre[mi];
-        const int tx = (v.cam.W + 31) >> 5;
-        const int x = (t % tx) * 32 + (threadIdx.x & 31);
-        const int y0 = (t / tx) * kStageTileH + (threadIdx.x >> 5);
-        float d[kStageTileH / 8];  // this thread's pixels (x, y0 + 8 r), depths loaded first
-#pragma unroll
-        for (int r = 0; r < kStageTileH / 8; ++r)
-            d[r] = x < v.cam.W && y0 + 8 * r < v.cam.H ? read_depth(v.in, x, y0 + 8 * r) : __int_as_float(0x7fffffff);
+        int x, y0;
+        const MapView& v = alloc_tile(views, pre, item, x, y0);
 #pragma unroll 1
-        for (int r = 0; r < kStageTileH / 8; ++r)
-            band_blocks_at(v, x, y0 + 8 * r, d[r], [&](unsigned long long key, int bx, int by, int bz) {
-                stage_block<kTileSet>(set, m, key, bx, by, bz);
-            });
+        for (int y = y0; y < y0 + kStageTileH; y += 8)
+            if (x < v.cam.W && y < v.cam.H)
+                band_blocks(v, x, y, [&](unsigned long long key, int bx, int by, int bz) {
+                    stage_block<kTileSet>(set, v.m, key, bx, by, bz);
+                });
         __syncthreads();
-        insert_staged<kTileSet>(set, m, threadIdx.x, blockDim.x);
+        insert_staged<kTileSet>(set, v.m, threadIdx.x, blockDim.x);
         __syncthreads();
     }
 }
@@ -138,9 +215,9 @@ __global__ void __launch_bounds__(256) reset_kernel(DevMap m, bool whole)
 
 // ------------------------------------------------------------------ launchers
 template <class V>
-cudaError_t launch_alloc(const V& views, int totalTiles, const Launcher& l, cudaStream_t s)
+cudaError_t launch_alloc(const V& views, int totalTiles, bool near, const Launcher& l, cudaStream_t s)
 {
-    return launch_stage<V>(alloc_kernel<V>, stage_grid(l, l.alloc, totalTiles), 256, s, views);
+    return launch_stage<V>(near ? alloc_kernel<V> : far_alloc<V>, stage_grid(l, l.alloc, totalTiles), 256, s, views);
 }
 
 template <class V>
@@ -162,8 +239,8 @@ cudaError_t launch_fuse(const V& views, int fmt, const Launcher& l, cudaStream_t
     }
 }
 
-template cudaError_t launch_alloc<OneView>(const OneView&, int, const Launcher&, cudaStream_t);
-template cudaError_t launch_alloc<ManyViews>(const ManyViews&, int, const Launcher&, cudaStream_t);
+template cudaError_t launch_alloc<OneView>(const OneView&, int, bool, const Launcher&, cudaStream_t);
+template cudaError_t launch_alloc<ManyViews>(const ManyViews&, int, bool, const Launcher&, cudaStream_t);
 template cudaError_t launch_visibility<OneView>(const OneView&, const Launcher&, cudaStream_t);
 template cudaError_t launch_visibility<ManyViews>(const ManyViews&, const Launcher&, cudaStream_t);
 template cudaError_t launch_fuse<OneView>(const OneView&, int, const Launcher&, cudaStream_t);

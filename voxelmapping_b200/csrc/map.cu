@@ -93,8 +93,8 @@ bool pose_ok(const double p[16])
 namespace vmapb {
 // How far the view's ray samples get from the world's origin on any axis, in
 // voxels: every sample lies between a ray's start and end, and the farthest of
-// these points belong to the image corners.
-static double view_reach(const vmap_map* m, const double pose[16])
+// these points belong to the image corners. (Or from the camera.)
+static double view_reach(const vmap_map* m, const double pose[16], bool from_camera = false)
 {
     const vmap_config& c = m->cfg;
     double reach = 0;
@@ -103,7 +103,7 @@ static double view_reach(const vmap_map* m, const double pose[16])
         const double x = ((k & 1 ? c.width : -1) - c.cx) / c.fx * z, y = ((k & 2 ? c.height : -1) - c.cy) / c.fy * z;
         for (int i = 0; i < 3; ++i) {
             const double* r = pose + 4 * i;
-            const double p = std::fabs(r[0] * x + r[1] * y + r[2] * z + r[3]) / c.voxel_size;
+            const double p = std::fabs(r[0] * x + r[1] * y + r[2] * z + (from_camera ? 0.0 : r[3])) / c.voxel_size;
             if (!std::isfinite(p)) return HUGE_VAL;
             reach = std::fmax(reach, p);
         }
@@ -159,6 +159,10 @@ void make_view(const vmap_map* m, const double pose[16], MapView& v)
     if (pose) {
         v.cam.tame = tame_view(m, v.Ti);
         const double reach = view_reach(m, pose);
+        // a band ends mu / 2 behind its depth
+        const double pos = std::fmax(std::fabs(pose[3]), std::fmax(std::fabs(pose[7]), std::fabs(pose[11]))) / m->cfg.voxel_size;
+        const double band = view_reach(m, pose, true) * (1.0 + m->cfg.truncation / (2.0 * kMaxDepth));
+        v.cam.near = v.cam.tame && m->cfg.fx > 1e-4f && m->cfg.fy > 1e-4f && pos + band < 0x1p20 && band < 8 * 510;
         v.out.wide = !m->dm.grid || !(reach < narrow_limit(m->dm.g));
         // a jump rounds a position by half a unit in the last place, 2^-24 of
         // it; a cube is crossed in some 50 jumps at most
@@ -495,6 +499,7 @@ vmap_status build_map(const vmap_config& cfg, unsigned char* base, cudaStream_t 
     m->dm.capacity = cfg.num_blocks;
     m->dm.blockBytes = (int)blockBytes;
     m->dm.vs = cfg.voxel_size;
+    m->dm.vsRcp = 1.f / cfg.voxel_size;
     m->dm.mu = cfg.truncation;
     m->dm.muRcp = 1.f / cfg.truncation;
     m->dm.wmax = (float)cfg.max_weight;
@@ -613,7 +618,7 @@ static vmap_status fuse_impl(vmap_map* m, const void* depth, int dtype, size_t d
     ov.queue = m->dm.ctr + C_RAYQ;
     const int tiles = stage_tiles(m->cfg.width, m->cfg.height);
     // alloc_kernel clears the visible counter the visibility kernel fills
-    VMAP_CK(staged(m, VMAP_STAGE_ALLOC, s, [&] { return launch_alloc(ov, tiles, m->launcher, s); }));
+    VMAP_CK(staged(m, VMAP_STAGE_ALLOC, s, [&] { return launch_alloc(ov, tiles, ov.v.cam.near != 0, m->launcher, s); }));
     VMAP_CK(staged(m, VMAP_STAGE_VISIBILITY, s, [&] { return launch_visibility(ov, m->launcher, s); }));
     VMAP_CK(staged(m, VMAP_STAGE_FUSE, s, [&] { return launch_fuse(ov, m->cfg.voxel_format, m->launcher, s); }));
     return VMAP_OK;

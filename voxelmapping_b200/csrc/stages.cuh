@@ -152,6 +152,75 @@ __device__ __forceinline__ void band_blocks(const MapView& v, int x, int y, Stag
     band_blocks_at(v, x, y, read_depth(v.in, x, y), stage);
 }
 
+// The same band for near views (CamParams::near), a whole warp together, one
+// pixel a lane (d NaN: no pixel). The walk has the reference's samples, sum for
+// sum, but no conversion instruction: voxel coordinates stay floats (whole
+// numbers below 2^21), truncation toward zero is an add of 1.5 * 2^23 with the
+// coordinate's sign, rounded toward zero, and a block number the low bits of a
+// multiply-add rounded down. A block is a 30-bit key relative to `base` (the
+// camera's block less 512 on each axis; no band of a near view gets farther
+// away); `stage(key)` is called with each key a lane's samples enter, less those
+// that the lane before it enters with the same sample.
+struct BandBase {
+    int x, y, z;
+};
+__device__ __forceinline__ BandBase band_base(const MapView& v)
+{
+    const float k = 0.125f * v.out.vsinv;
+    return BandBase{__float2int_rd(v.T.m[0][3] * k) - 512, __float2int_rd(v.T.m[1][3] * k) - 512,
+                    __float2int_rd(v.T.m[2][3] * k) - 512};
+}
+
+template <class Stage>
+__device__ __forceinline__ void band_keys(const MapView& v, const BandBase& base, int x, int y, float d, int lane,
+                                          Stage stage)
+{
+    const DevMap& m = v.m;
+    constexpr float M = 12582912.f;  // 1.5 * 2^23
+    constexpr unsigned full = 0xffffffffu;
+    auto block = [](float p) {  // block number of the truncated coordinate, plus M's bits
+        const float sm = copysignf(M, p);
+        return __float_as_int(__fmaf_rd(__fsub_rn(__fadd_rz(p, sm), sm), 0.125f, M));
+    };
+    const float tdh = __fmul_rn(m.mu, 0.5f);
+    const float dn = fmaxf(kMinDepth, __fsub_rn(d, tdh));
+    const float df = fmaxf(kMinDepth, __fadd_rn(d, tdh));
+    int n = 0;
+    float px = 0.f, py = 0.f, pz = 0.f, dx = 0.f, dy = 0.f, dz = 0.f;
+    if (d >= kMinDepth && d <= kMaxDepth && dn < df) {
+        auto voxel = [&](float w) { return __fsub_rn(__fadd_rd(div_exact(w, m.vs, m.vsRcp), M), M); };  // floor(w / vs)
+        const float3 a = unproject(x, y, dn, v.cam.ifx, v.cam.ify, v.cam.cx, v.cam.cy);
+        const float3 wa = xf_apply(v.T, a.x, a.y, a.z);
+        const float3 b = unproject(x, y, df, v.cam.ifx, v.cam.ify, v.cam.cx, v.cam.cy);
+        const float3 wb = xf_apply(v.T, b.x, b.y, b.z);
+        px = voxel(wa.x);
+        py = voxel(wa.y);
+        pz = voxel(wa.z);
+        const float3 dir = make_float3(__fsub_rn(voxel(wb.x), px), __fsub_rn(voxel(wb.y), py), __fsub_rn(voxel(wb.z), pz));
+        const float c = __fadd_ru(__fmul_rn(2.f, __fsqrt_rn(sqnorm(dir))), 8388608.f);  // ceil(2 len) + 2^23
+        n = __float_as_int(c) - 0x4B000000;
+        const float den = __fsub_rn(__fsub_rn(c, 8388608.f), 1.f), rd = rcp_newton(den);
+        dx = div_exact(dir.x, den, rd);
+        dy = div_exact(dir.y, den, rd);
+        dz = div_exact(dir.z, den, rd);
+    }
+    constexpr unsigned mb = 0x4B400000u;
+    const unsigned off = mb + (mb << 10) + (mb << 20) + base.x + (base.y << 10) + (base.z << 20);
+    const int most = __reduce_max_sync(full, n);
+    unsigned last = ~0u;
+#pragma unroll 1
+    for (int s = 0; s < most; ++s) {
+        unsigned key = (unsigned)((block(pz) * 1024 + block(py)) * 1024 + block(px)) - off;
+        if (s >= n) key = last;
+        const unsigned before = __shfl_up_sync(full, key, 1);
+        if (key != last && (lane == 0 || before != key)) stage(key);
+        last = key;
+        px = __fadd_rn(px, dx);
+        py = __fadd_rn(py, dy);
+        pz = __fadd_rn(pz, dz);
+    }
+}
+
 // ---------------------------------------------------------------- visibility
 // checkBlockVisible over allocated blocks [32 g, 32 g + 32) of one map, one
 // warp (every lane calls): visible slots are appended to the map's visible

@@ -82,6 +82,7 @@ struct DevMap {
     int capacity;
     int blockBytes;
     float vs;   // voxel size
+    float vsRcp; // 1.f / vs
     float mu;   // truncation distance
     float muRcp; // 1.f / mu
     float wmax; // weight cap
@@ -610,6 +611,7 @@ struct CamParams {
     float ifx, ify;  // (float)(1.0 / (double)f), as the reference's host code
     float fW, fH;    // W, H
     int tame;        // projections of any block overflow nothing, pixels below 2^22 (project_tame)
+    int near;        // and every depth band stays below 2^20 voxels and within 510 blocks of the camera's (band_keys)
 };
 
 struct FrameIn {

@@ -106,7 +106,7 @@ cudaError_t launch_stage(void (*kernel)(KArgs...), int grid, int block, cudaStre
 
 // fusion.cu
 template <class V>
-cudaError_t launch_alloc(const V& views, int totalTiles, const Launcher& l, cudaStream_t s);
+cudaError_t launch_alloc(const V& views, int totalTiles, bool near, const Launcher& l, cudaStream_t s);  // near: every view is
 template <class V>
 cudaError_t launch_visibility(const V& views, const Launcher& l, cudaStream_t s);
 template <class V>
