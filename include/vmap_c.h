@@ -278,8 +278,8 @@ typedef struct vmap_launch_config {
     int normals_ctas_per_sm;
     int mesh_ctas_per_sm;
     /* order in which the ray marcher hands out each image's pixel tiles:
-     * 0 = default (bottom rows first), 1 = top rows first, 2 = alternating
-     * from both ends. Tiles are independent, so only the time changes: the
+     * 0 = default (alternating from both ends), 1 = top rows first, 2 =
+     * alternating from both ends. Tiles are independent, so only the time changes: the
      * slowest tiles are best started first. */
     int raycast_tile_order;
     /* ray-marcher tile: a warp marches a tile of 32 neighbouring rays,

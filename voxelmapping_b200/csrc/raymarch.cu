@@ -25,10 +25,8 @@
 //
 // Scheduling: the kernel is persistent. Each warp takes 8x4-pixel tiles from
 // one device-side queue shared by every map of the batch until it runs dry.
-// A map's tiles are handed out in a selectable order: starting with the
-// slowest tiles shortens the tail of the launch (bottom rows first measured
-// 5 % faster than top rows first on the room sequences, whose lower rows see
-// the floor and the nearest surfaces).
+// A map's tiles are handed out in a selectable order, alternating from both
+// ends of the image by default (march_tile).
 // (Refilling lanes from a larger group as their rays finish was measured
 // 2.8x slower: lanes at different depths scatter their loads and lookups.)
 #include "march.cuh"
