@@ -318,8 +318,9 @@ class HostPipeline:
         f.pose[:] = [float(x) for x in np.asarray(pose, np.float64).reshape(16)]
         out = None
         if render:
-            v = torch.empty((vm.height, vm.width, 4), dtype=torch.float32).pin_memory()
-            n = torch.empty_like(v).pin_memory() if self.normals else None
+            # pinned from the start: .pin_memory() would copy the 4.9 MB (640x480) of an uninitialised pageable array
+            v = torch.empty((vm.height, vm.width, 4), dtype=torch.float32, pin_memory=True)
+            n = torch.empty((vm.height, vm.width, 4), dtype=torch.float32, pin_memory=True) if self.normals else None
             f.vmap_host = v.data_ptr()
             f.nmap_host = n.data_ptr() if n is not None else None
             out = (v.numpy(), n.numpy() if n is not None else None)
