@@ -24,7 +24,7 @@ __device__ __forceinline__ float3 fma3(float k, float3 d, float3 r)
 // Per-lane state of one ray. cx, cy, cz: floor codes (March::fl) of a voxel in
 // the region that the last lookup settled: the aligned cube of side cmask + 1
 // voxels, 8 (one block) with its slot in cblk, or 8, 32 or 128 that hold no
-// allocated block (cblk -1). bits: occupancy word of that voxel's brick.
+// allocated block (cblk -1).
 struct Ray {
     int x, y;
     float3 res, dir, inv;
@@ -32,7 +32,6 @@ struct Ray {
     float sdf;
     bool valid;
     int cx, cy, cz, cmask, cblk;
-    unsigned long long bits;
 };
 
 // WIDE: some ray of the view may leave the narrow range (narrow_limit, set per
@@ -139,13 +138,14 @@ struct March {
         return c;
     }
 
-    // Slot of the block that holds the far corners when they leave corner 0's
-    // block `slot` on exactly one axis, `slot` itself when they do not leave
-    // it: read together with the sample, so the corners' own reads need not
-    // wait for it.
+    // Slot of the block of the farthest corner, past every axis on which the
+    // corners leave corner 0's block `slot` (not for all three; `slot` itself
+    // when they do not leave it): read together with the sample, so that the
+    // corners' own reads need not wait for it and the other links of the block
+    // are at hand.
     static __device__ __forceinline__ int far_slot(const DevMap& m, int slot, int cross)
     {
-        return cross == 1 || cross == 2 || cross == 4 ? ld_map<NC>(m.nbr + (6 * (size_t)slot + cross - 1)) : slot;
+        return cross && cross < 7 ? ld_map<NC>(m.nbr + (6 * (size_t)slot + cross - 1)) : slot;
     }
 
     // Whether all 8 words are observed, by their smallest weight: the weight is
@@ -173,8 +173,8 @@ struct March {
     static __device__ __forceinline__ bool corners8(const DevMap& m, int slot, int far, int cross, const Corners& c, Word w0,
                                                     float* s)
     {
-        bool ok, v;
-        s[0] = value(w0, ok);
+        Word w[8];
+        w[0] = w0;
         if (cross == 0 || cross == 1 || cross == 2 || cross == 4) {
             const bool gone = far < 0;  // the far corners' block is not allocated
             const long long hop = gone ? 0ll : (long long)(far - slot) * m.blockBytes;
@@ -183,46 +183,47 @@ struct March {
             const long long dy = ((c.y1 & 7) - (c.y0 & 7)) * 8 * (int)sizeof(Word) + (cross == 2 ? hop : 0ll);
             const long long dz = ((c.z1 & 7) - (c.z0 & 7)) * 64 * (int)sizeof(Word) + (cross == 4 ? hop : 0ll);
             auto ld = [](const char* p) { return ld_map<NC>(reinterpret_cast<const Word*>(p)); };
-            const Word w1 = ld(ax), w2 = ld(a + dy), w3 = ld(ax + dy), w4 = ld(a + dz), w5 = ld(ax + dz);
-            const Word w6 = ld(a + dy + dz), w7 = ld(ax + dy + dz);
-            if (!gone && all_observed(w0, w1, w2, w3, w4, w5, w6, w7)) {  // most reads
-                s[0] = F::tsdf(w0);
-                s[1] = F::tsdf(w1);
-                s[2] = F::tsdf(w2);
-                s[3] = F::tsdf(w3);
-                s[4] = F::tsdf(w4);
-                s[5] = F::tsdf(w5);
-                s[6] = F::tsdf(w6);
-                s[7] = F::tsdf(w7);
-                return true;
-            }
-            s[1] = value(w1, v); ok &= v;
-            s[2] = value(w2, v); ok &= v;
-            s[3] = value(w3, v); ok &= v;
-            s[4] = value(w4, v); ok &= v;
-            s[5] = value(w5, v); ok &= v;
-            s[6] = value(w6, v); ok &= v;
-            s[7] = value(w7, v); ok &= v;
+            w[1] = ld(ax);
+            w[2] = ld(a + dy);
+            w[3] = ld(ax + dy);
+            w[4] = ld(a + dz);
+            w[5] = ld(ax + dz);
+            w[6] = ld(a + dy + dz);
+            w[7] = ld(ax + dy + dz);
             if (gone) {
 #pragma unroll
                 for (int k = 1; k < 8; ++k)
-                    if (k & cross) s[k] = 1.f;
-                ok = false;
+                    if (k & cross) w[k] = Word();
             }
-        } else {  // several axes: independent links, then independent corners
+        } else {
+            // several axes: independent links, then independent corners, with
+            // no branch a corner (each had two, run by some lane of half of
+            // the warp's iterations); corners without a block read corner 0
             const int* L = m.nbr + 6 * (size_t)slot;
+            int to[8];
+#pragma unroll
+            for (int k = 1; k < 8; ++k) {
+                const int o = k & cross;  // corner k's block, as an offset from corner 0's
+                const int link = ld_map<NC>(L + (o && o < 7 ? o - 1 : 0));
+                to[k] = o == cross ? far : o ? link : slot;
+            }
+            if (cross == 7) to[7] = find(m, c.x1, c.y1, c.z1);  // no link to the far one on all axes
 #pragma unroll
             for (int k = 1; k < 8; ++k) {
                 const int vx = (k & 1) ? c.x1 : c.x0, vy = (k & 2) ? c.y1 : c.y0, vz = (k & 4) ? c.z1 : c.z0;
-                const int o = k & cross;  // corner k's block, as an offset from corner 0's
-                int at_slot = slot;
-                if (k == 7 && o == 7) at_slot = find(m, vx, vy, vz);  // no link to the far one on all axes
-                else if (o) at_slot = ld_map<NC>(L + o - 1);
-                s[k] = voxel(m, at_slot, vx, vy, vz, v);
-                ok &= v;
+                w[k] = ld_map<NC>(Layout<FMT>::words(m, to[k] < 0 ? slot : to[k]) + at(vx, vy, vz));
+                if (to[k] < 0) w[k] = Word();
             }
         }
-        return ok;
+        if (all_observed(w[0], w[1], w[2], w[3], w[4], w[5], w[6], w[7])) {  // most reads
+#pragma unroll
+            for (int k = 0; k < 8; ++k) s[k] = F::tsdf(w[k]);
+            return true;
+        }
+        bool v;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) s[k] = value(w[k], v);
+        return false;
     }
 
     // Every 1-voxel step inside the unallocated block (bx, by, bz) reads
@@ -322,7 +323,6 @@ struct March {
         r.cx = r.cy = r.cz = INT_MIN;  // a region of its own: no sample's codes have this top bit
         r.cmask = 7;
         r.cblk = -1;
-        r.bits = 0ull;
         return true;
     }
 
@@ -334,10 +334,10 @@ struct March {
     }
 
     // Looks the voxel up: the largest empty cube the occupancy words show
-    // around it, or its block's slot. Within the brick of the last lookup its
-    // word is at hand and an empty block needs no read; in a new brick the
-    // three reads do not depend on one another.
-    static __device__ __forceinline__ void settle(const DevMap& m, Ray& r, int ix, int iy, int iz, bool same_brick)
+    // around it, or its block's slot. The three reads do not depend on one
+    // another (the brick's word kept from the last lookup spared two of them at
+    // the price of branches, and was slower).
+    static __device__ __forceinline__ void settle(const DevMap& m, Ray& r, int ix, int iy, int iz)
     {
         if (WIDE && !m.grid) {
             r.cmask = 7;
@@ -345,17 +345,10 @@ struct March {
             return;
         }
         const int brick8 = grid_brick8(m, ix, iy, iz), bit8 = grid_bit8(ix, iy, iz);
-        const unsigned long long* cell = grid_cell(m, brick8, bit8);
-        unsigned long long e = 0ull;
-        r.cmask = 7;
-        if (same_brick) {
-            if ((r.bits >> (bit8 >> 3)) & 1ull) e = ld_map<NC>(cell);
-        } else {
-            const unsigned long long above = ld_map<NC>(m.occ2 + grid_region(m, ix, iy, iz));
-            r.bits = ld_map<NC>(grid_occ(m, brick8));
-            e = ld_map<NC>(cell);
-            if (r.bits == 0ull) r.cmask = above == 0ull ? 127 : 31;
-        }
+        const unsigned long long above = ld_map<NC>(m.occ2 + grid_region(m, ix, iy, iz));
+        const unsigned long long here = ld_map<NC>(grid_occ(m, brick8));
+        const unsigned long long e = ld_map<NC>(grid_cell(m, brick8, bit8));
+        r.cmask = here ? 7 : above ? 31 : 127;
         r.cblk = slot_of(m, e, ix, iy, iz);
     }
 
@@ -397,7 +390,7 @@ struct March {
             r.cx = ix;
             r.cy = iy;
             r.cz = iz;
-            if (d & ~r.cmask) settle(v.m, r, ix, iy, iz, !(d & ~31));
+            if (d & ~r.cmask) settle(v.m, r, ix, iy, iz);
             if (r.cblk >= 0) return kBlock;
             const float run = run_limit(r, v.out.slack);
             do empty_jump(r);
@@ -435,8 +428,7 @@ struct March {
             ds = __fadd_rn(ds, 1.f);
             const int ix = fl(q.x), iy = fl(q.y), iz = fl(q.z);
             ok[k] = ds < r.dist_lim && !(moved(r, ix, iy, iz) & ~7);
-            w[k] = Word();
-            if (ok[k]) w[k] = ld_map<NC>(blk + at(ix, iy, iz));
+            w[k] = ld_map<NC>(blk + at(ix, iy, iz));  // (some voxel of the block where the sample is not in it)
         }
         int n = 1;  // samples consumed: this one, then the leading unobserved ones ahead
         bool run = true;

@@ -15,13 +15,13 @@
 //     occupancy words, so that the jumps inside one need no lookup either;
 //   * the trilinear corners of all rays of a warp are read together, whether
 //     they lie in one block or two.
-// What bounds it: the instructions (a third to a half of them on the ALU pipe,
-// which runs at half rate: at 640x480 the kernel issues 70 % of the time while
-// all its warps run) and, in scenes seen at grazing angles, the slowest tiles'
-// latency. Against a lookup per block through a warp-shared cache and the hash
-// table, event time of the launch, three rooms each: 48 -> 30 us at 160x120 /
-// 16 mm, 63 -> 39 at 320x240 / 8 mm, 96 -> 70 at 640x480 / 5 mm, 293 -> 241 at
-// 1280x720 / 4 mm, 320 -> 131 for an 800x600 full march (raycast_mode 1).
+// What bounds it: the instructions and branches (at 640x480 the kernel issues
+// 70 % of the time while all its warps run) and, in scenes seen at grazing
+// angles, the slowest tiles' latency. Against a lookup per block through a
+// warp-shared cache and the hash table, event time of the launch, three rooms
+// each: 48 -> 26 us at 160x120 / 16 mm, 63 -> 32 at 320x240 / 8 mm, 96 -> 58 at
+// 640x480 / 5 mm, 293 -> 208 at 1280x720 / 4 mm, 97 -> 50 a view at 517x389,
+// 320 -> 108 for an 800x600 full march (raycast_mode 1).
 //
 // Scheduling: the kernel is persistent. Each warp takes 8x4-pixel tiles from
 // one device-side queue shared by every map of the batch until it runs dry.
