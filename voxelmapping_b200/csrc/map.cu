@@ -139,8 +139,6 @@ void make_view(const vmap_map* m, const double pose[16], MapView& v)
     v.cam.cy = m->cfg.cy;
     v.cam.ifx = (float)(1.0 / (double)m->cfg.fx);
     v.cam.ify = (float)(1.0 / (double)m->cfg.fy);
-    v.cam.fW = (float)m->cfg.width;
-    v.cam.fH = (float)m->cfg.height;
     v.in.active = 1;
     v.in.dscale = 1.f;
     if (pose) {

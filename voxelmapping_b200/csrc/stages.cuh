@@ -25,14 +25,16 @@ __device__ __forceinline__ unsigned small_floor(float x) { return __float_as_uin
 
 // ---------------------------------------------------------------- frames
 // Depth and colour frames are inputs: nothing writes them while a kernel runs.
+// A pixel's place is never negative: unsigned, its 64-bit address needs no sign
+// extensions.
 template <int DT>
 __device__ __forceinline__ float read_depth_t(const FrameIn& f, int x, int y)
 {
-    const char* row = reinterpret_cast<const char*>(f.depth) + (size_t)y * f.dpitch;
+    const char* row = reinterpret_cast<const char*>(f.depth) + (size_t)(unsigned)y * f.dpitch;
     if constexpr (DT == VMAP_DEPTH_F32) {
-        return __ldg(reinterpret_cast<const float*>(row) + x);
+        return __ldg(reinterpret_cast<const float*>(row) + (unsigned)x);
     } else {
-        return __fmul_rn(small_to_float(__ldg(reinterpret_cast<const unsigned short*>(row) + x)), f.dscale);
+        return __fmul_rn(small_to_float(__ldg(reinterpret_cast<const unsigned short*>(row) + (unsigned)x)), f.dscale);
     }
 }
 
@@ -334,7 +336,8 @@ __device__ __forceinline__ bool project_tame(const MapView& v, int vx0, float wy
     }
 #pragma unroll
     for (int a = 0; a < 2; ++a) {  // image columns, then rows
-        const float f = a ? v.cam.fy : v.cam.fx, c = a ? v.cam.cy : v.cam.cx, end = a ? v.cam.fH : v.cam.fW;
+        const float f = a ? v.cam.fy : v.cam.fx, c = a ? v.cam.cy : v.cam.cx;
+        const unsigned end = a ? v.cam.H : v.cam.W;
         float q[NV];
         row(a, q);
 #pragma unroll
@@ -343,8 +346,9 @@ __device__ __forceinline__ bool project_tame(const MapView& v, int vx0, float wy
 #pragma unroll
         for (int x = 0; x < NV; ++x) {
             const float i = __fadd_rn(__fadd_rn(q[x], c), 0.5f);
-            in[x] = (a ? in[x] : true) && i >= 0.f && i < end;
-            (a ? pv : pu)[x] = (int)(small_floor(i) - 0x4B000000u);
+            const unsigned at = small_floor(i) - 0x4B000000u;  // 2^22 or more for any i outside [0, 2^22), NaN included
+            in[x] = (a ? in[x] : true) && at < end;
+            (a ? pv : pu)[x] = (int)at;
         }
     }
     return true;
@@ -425,7 +429,7 @@ __device__ __forceinline__ void fuse_block(const MapView& v, int slot, int v0)
         for (int x = 0; x < NV; ++x) {
             pix[x] = 0u;
             if (ok[x]) {
-                const uint8_t* px = v.in.rgb + (size_t)pv[x] * v.in.rgbPitch + 3 * pu[x];
+                const uint8_t* px = v.in.rgb + (size_t)(unsigned)pv[x] * v.in.rgbPitch + (size_t)(unsigned)pu[x] * 3;
                 pix[x] = (unsigned)__ldg(px) | ((unsigned)__ldg(px + 1) << 8) | ((unsigned)__ldg(px + 2) << 16);
             }
         }

@@ -609,7 +609,6 @@ struct CamParams {
     int W, H;
     float fx, fy, cx, cy;
     float ifx, ify;  // (float)(1.0 / (double)f), as the reference's host code
-    float fW, fH;    // W, H
     int tame;        // projections of any block overflow nothing, pixels below 2^22 (project_tame)
     int near;        // and every depth band stays below 2^20 voxels and within 510 blocks of the camera's (band_keys)
 };
