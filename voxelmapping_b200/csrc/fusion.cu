@@ -169,6 +169,10 @@ __global__ void __launch_bounds__(256) visibility_kernel(V views)
 // pixel's range checked by one unsigned comparison and unsigned addresses to
 // 41.4 and 130 us. Prefetching the voxel words, or the next block's, into L2
 // changes nothing or costs up to 7 us: the loads' latency is not what bounds it.
+// Several maps: the view's fields are loaded and take registers, and reading a
+// pixel's colour in two loads instead of three spills less (4 to 28 B instead
+// of 28 to 108) and is faster, 2702 -> 2673 us for a step of 32 maps at 640x480
+// with their rendering; for one map it is slower (FP16 at 1280x720: 130 -> 140).
 // A team of 512 / kFuseVoxels threads per visible block, kFuseVoxels voxels
 // of an x-row per thread; 256 / team blocks per CTA, grid-stride over the
 // visible blocks of all maps. 6 resident CTAs per SM (at most 40 registers)
@@ -191,7 +195,7 @@ __global__ void __launch_bounds__(256, 6) fuse_kernel(V views)
     for (int i = blockIdx.x * teams + team; i < total; i += gridDim.x * teams) {
         const int mi = map_of(pre, nmaps, i);
         const MapView& v = views[mi];
-        fuse_voxels<FMT, kFuseVoxels>(v, v.m.visList[i - pre[mi]], v0);
+        fuse_voxels<FMT, kFuseVoxels, V::kMany>(v, v.m.visList[i - pre[mi]], v0);
     }
 }
 

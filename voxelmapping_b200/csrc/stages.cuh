@@ -381,7 +381,7 @@ __device__ __forceinline__ unsigned blend2(unsigned c, unsigned pa, unsigned pb,
 // the surface or outside the frame move no voxel bytes. Nothing is written
 // unless a voxel updates. A voxel's first update is the running average with
 // weight 0 of a zero TSDF, (0 * 0 + sdf) / 1.
-template <int FMT, bool COLOR, int DT, int NV = 4>
+template <int FMT, bool COLOR, int DT, int NV = 4, bool PAIR = false>
 __device__ __forceinline__ void fuse_block(const MapView& v, int slot, int v0)
 {
     typedef Layout<FMT> L;
@@ -430,7 +430,13 @@ __device__ __forceinline__ void fuse_block(const MapView& v, int slot, int v0)
             pix[x] = 0u;
             if (ok[x]) {
                 const uint8_t* px = v.in.rgb + (size_t)(unsigned)pv[x] * v.in.rgbPitch + (size_t)(unsigned)pu[x] * 3;
-                pix[x] = (unsigned)__ldg(px) | ((unsigned)__ldg(px + 1) << 8) | ((unsigned)__ldg(px + 2) << 16);
+                if constexpr (PAIR) {  // the two bytes at the even address and the third: any alignment, no byte more
+                    const unsigned odd = (unsigned)(size_t)px & 1u;
+                    const unsigned two = __ldg(reinterpret_cast<const unsigned short*>(px + odd)), one = __ldg(odd ? px : px + 2);
+                    pix[x] = __byte_perm(two, one, odd ? 0x7104 : 0x7410);
+                } else {
+                    pix[x] = (unsigned)__ldg(px) | ((unsigned)__ldg(px + 1) << 8) | ((unsigned)__ldg(px + 2) << 16);
+                }
             }
         }
     }
@@ -465,16 +471,16 @@ __device__ __forceinline__ void fuse_block(const MapView& v, int slot, int v0)
 
 // fuse_block for the frame's depth type; colour when the frame carries it
 // (the map must keep colour).
-template <int FMT, int NV = 4>
+template <int FMT, int NV = 4, bool PAIR = false>
 __device__ __forceinline__ void fuse_voxels(const MapView& v, int slot, int v0)
 {
     const bool color = v.in.rgb != nullptr;
     if (v.in.dtype == VMAP_DEPTH_U16) {
-        if (color) fuse_block<FMT, true, VMAP_DEPTH_U16, NV>(v, slot, v0);
-        else fuse_block<FMT, false, VMAP_DEPTH_U16, NV>(v, slot, v0);
+        if (color) fuse_block<FMT, true, VMAP_DEPTH_U16, NV, PAIR>(v, slot, v0);
+        else fuse_block<FMT, false, VMAP_DEPTH_U16, NV, PAIR>(v, slot, v0);
     } else {
-        if (color) fuse_block<FMT, true, VMAP_DEPTH_F32, NV>(v, slot, v0);
-        else fuse_block<FMT, false, VMAP_DEPTH_F32, NV>(v, slot, v0);
+        if (color) fuse_block<FMT, true, VMAP_DEPTH_F32, NV, PAIR>(v, slot, v0);
+        else fuse_block<FMT, false, VMAP_DEPTH_F32, NV, PAIR>(v, slot, v0);
     }
 }
 

@@ -656,6 +656,7 @@ struct MapView {
 constexpr int kMaxBatch = 256;
 
 struct OneView {
+    static constexpr bool kMany = false;
     MapView v;
     unsigned* queue;  // work-queue counters of this step
     __device__ __forceinline__ int count() const { return 1; }
@@ -663,6 +664,7 @@ struct OneView {
 };
 
 struct ManyViews {
+    static constexpr bool kMany = true;
     const MapView* v;
     int n;
     unsigned* queue;
