@@ -171,7 +171,7 @@ __global__ void __launch_bounds__(256) visibility_kernel(V views)
 // changes nothing or costs up to 7 us: the loads' latency is not what bounds it.
 // Several maps: the view's fields are loaded and take registers, and reading a
 // pixel's colour in two loads instead of three spills less (4 to 28 B instead
-// of 28 to 108) and is faster, 2702 -> 2673 us for a step of 32 maps at 640x480
+// of 28 to 108) and is faster, 2699 -> 2668 us for a step of 32 maps at 640x480
 // with their rendering; for one map it is slower (FP16 at 1280x720: 130 -> 140).
 // A team of 512 / kFuseVoxels threads per visible block, kFuseVoxels voxels
 // of an x-row per thread; 256 / team blocks per CTA, grid-stride over the
