@@ -163,7 +163,8 @@ void make_view(const vmap_map* m, const double pose[16], MapView& v)
         v.cam.near = v.cam.tame && m->cfg.fx > 1e-4f && m->cfg.fy > 1e-4f && pos + band < 0x1p20 && band < 8 * 510;
         v.out.wide = !m->dm.grid || !(reach < narrow_limit(m->dm.g));
         // a jump rounds a position by half a unit in the last place, 2^-24 of
-        // it; a cube is crossed in some 50 jumps at most
+        // it; the 48 block faces of the widest cube take at most 96 jumps (one
+        // that stops short of a face is followed by a step of one voxel)
         v.out.slack = (float)(0.05 + reach * 0x1p-17);
     }
     v.out.mode = m->cfg.raycast_mode;

@@ -353,17 +353,22 @@ struct March {
     }
 
     // Ray distance up to which a ray at res is certain to stay in its empty
-    // cube: the exit distance less a margin for the rounding of the jumps'
-    // positions. (Wide views look at every position instead.)
+    // cube: the exit distance from the cube with its exit faces drawn in by
+    // `slack` voxels, the rounding of the positions on the way. (A margin on
+    // the distance would not do: a ray of slope s to a face that is off by e
+    // reaches it e / s early. The entry faces need none: a rounded step never
+    // goes back.) A ray that starts within the slack looks its next position
+    // up. (Wide views look at every position instead.)
     static __device__ __forceinline__ float run_limit(const Ray& r, float slack)
     {
         if constexpr (WIDE) return r.dist_s;
-        auto exit = [&r](int i, float p, float d, float inv) {
-            return (ff(i & ~r.cmask) + (signbit(d) ? 0.f : (float)(r.cmask + 1)) - p) * inv;
+        const float far = (float)(r.cmask + 1) - slack;
+        auto exit = [&](int i, float p, float d, float inv) {
+            return (ff(i & ~r.cmask) + (signbit(d) ? slack : far) - p) * inv;
         };
         const float t = fminf(fminf(exit(r.cx, r.res.x, r.dir.x, r.inv.x), exit(r.cy, r.res.y, r.dir.y, r.inv.y)),
                               exit(r.cz, r.res.z, r.dir.z, r.inv.z));
-        return fminf(r.dist_lim, r.dist_s + t - slack);
+        return fminf(r.dist_lim, r.dist_s + t);
     }
 
     // First half of a loop iteration: from the sample at res towards the first
