@@ -81,7 +81,7 @@ __global__ void rebuild_hash_kernel(DevMap m, unsigned n, unsigned flags)
 {
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         m.ctr[C_ALLOC] = n;
-        m.ctr[C_UNKNOWN] = 0u;  // the copies before this kernel are done: [0, n) is what the pool holds
+        m.ctr[C_UNKNOWN] = 0u;  // the copies before this kernel are done, and all beyond [0, n) is clear
         if (flags) atomicOr(m.ctr + C_ERR, flags);
     }
     for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
@@ -193,11 +193,13 @@ vmap_status vmap_snapshot_load(vmap_map* map, const void* src, uint64_t bytes, v
                                               " blocks exceed the pool capacity of " + std::to_string(m.capacity));
     const uint32_t n = h.n_blocks;
     const unsigned char* p = static_cast<const unsigned char*>(src);
-    // a reset after a load that stopped half-way clears the whole pool
+    // blocks that may hold data: after a load that stopped half-way, any of the
+    // pool (until a load or a reset has cleared it)
+    const uint32_t used = map_pool_unknown(map) ? (uint32_t)m.capacity : st.allocated_blocks;
     SNAP_CK(cudaMemsetAsync(m.ctr + C_UNKNOWN, 1, sizeof(unsigned), s));
     // blocks beyond the snapshot must read as unobserved (zero) once handed out again
-    if (st.allocated_blocks > n)
-        SNAP_CK(cudaMemsetAsync(m.pool + (size_t)n * m.blockBytes, 0, (size_t)(st.allocated_blocks - n) * m.blockBytes, s));
+    if (used > n)
+        SNAP_CK(cudaMemsetAsync(m.pool + (size_t)n * m.blockBytes, 0, (size_t)(used - n) * m.blockBytes, s));
     SNAP_CK(cudaMemsetAsync(m.ctr, 0, C_UNKNOWN * sizeof(unsigned), s));
     clear_index_kernel<<<grid_for((size_t)m.nBucket * kSlots), 256, 0, s>>>(m);
     SNAP_CK(cudaGetLastError());

@@ -133,6 +133,7 @@ cudaError_t launch_export(const DevMap& m, int fmt, bool color, int first, int c
 // map.cu: device view of a map and the text behind vmap_last_error().
 const DevMap& map_device_view(const vmap_map* m);
 int map_device(const vmap_map* m);  // CUDA device the map was created on
+bool map_pool_unknown(const vmap_map* m);  // C_UNKNOWN as the last vmap_get_stats read it
 void set_last_error(const std::string& msg);
 
 // Allocation and normal-map kernels work on 32 x kStageTileH-pixel tiles, one
