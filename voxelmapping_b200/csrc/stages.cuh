@@ -166,6 +166,14 @@ __device__ __forceinline__ void band_blocks(const MapView& v, int x, int y, Stag
 struct BandBase {
     int x, y, z;
 };
+// Key of block numbers that each carry the bits of 1.5 * 2^23 or of a base below
+// them: keys wrap around 2^32, and the difference of two is exact.
+__host__ __device__ constexpr unsigned band_key(unsigned x, unsigned y, unsigned z) { return x + (y << 10) + (z << 20); }
+constexpr unsigned kBandBits = 0x4B400000u;  // 1.5 * 2^23 as a float
+static_assert(band_key(kBandBits - 4000u, kBandBits + 77u, kBandBits + 200000u) -
+                      band_key(kBandBits - 4512u, kBandBits - 435u, kBandBits + 199489u) ==
+                  (512u | 512u << 10 | 511u << 20),
+              "no signed overflow, which a constant expression refuses, and no carry between axes");
 __device__ __forceinline__ BandBase band_base(const MapView& v)
 {
     const float k = 0.125f * v.out.vsinv;
@@ -182,7 +190,7 @@ __device__ __forceinline__ void band_keys(const MapView& v, const BandBase& base
     constexpr unsigned full = 0xffffffffu;
     auto block = [](float p) {  // block number of the truncated coordinate, plus M's bits
         const float sm = copysignf(M, p);
-        return __float_as_int(__fmaf_rd(__fsub_rn(__fadd_rz(p, sm), sm), 0.125f, M));
+        return __float_as_uint(__fmaf_rd(__fsub_rn(__fadd_rz(p, sm), sm), 0.125f, M));
     };
     const float tdh = __fmul_rn(m.mu, 0.5f);
     const float dn = fmaxf(kMinDepth, __fsub_rn(d, tdh));
@@ -206,13 +214,12 @@ __device__ __forceinline__ void band_keys(const MapView& v, const BandBase& base
         dy = div_exact(dir.y, den, rd);
         dz = div_exact(dir.z, den, rd);
     }
-    constexpr unsigned mb = 0x4B400000u;
-    const unsigned off = mb + (mb << 10) + (mb << 20) + base.x + (base.y << 10) + (base.z << 20);
+    const unsigned off = band_key(kBandBits + (unsigned)base.x, kBandBits + (unsigned)base.y, kBandBits + (unsigned)base.z);
     const int most = __reduce_max_sync(full, n);
     unsigned last = ~0u;
 #pragma unroll 1
     for (int s = 0; s < most; ++s) {
-        unsigned key = (unsigned)((block(pz) * 1024 + block(py)) * 1024 + block(px)) - off;
+        unsigned key = band_key(block(px), block(py), block(pz)) - off;
         if (s >= n) key = last;
         const unsigned before = __shfl_up_sync(full, key, 1);
         if (key != last && (lane == 0 || before != key)) stage(key);
