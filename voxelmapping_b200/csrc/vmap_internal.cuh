@@ -114,9 +114,11 @@ __device__ __forceinline__ float div_exact(float a, float b, float y)
     return __fmaf_rn(__fmaf_rn(-b, q, a), y, q);
 }
 
-// 1 / b for normal b: the approximate reciprocal (within one unit in the last
-// place) and one Newton step, which rounds it correctly unless b's mantissa is
-// all ones (Markstein 1990), and to within 2^-24 (1 + 2^-23) then.
+// 1 / b, correctly rounded, for b whose reciprocal is normal (up to 2^126): the
+// approximate reciprocal (within one unit in the last place) and one Newton step.
+// The step is proven to round correctly unless b's mantissa is all ones
+// (Markstein 1990), where an approximation one unit low would stay as it is. The
+// hardware's is not low there: a test runs all 2^23 mantissas.
 __device__ __forceinline__ float rcp_newton(float b)
 {
     float y;
