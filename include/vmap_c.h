@@ -266,9 +266,9 @@ vmap_status vmap_batch_stall_probe(vmap_batch* batch, const vmap_batch_frame* fr
  * items, so any shape gives the same results and only the time changes.
  * 0 in a field selects the library default (alloc 8, visibility 2, fuse 16,
  * zrange 4, normals 8, mesh 8; raycast 0 = as many CTAs as fit on an SM, the
- * ray marcher being persistent). Values above 64 (tile orders above 2) are
- * refused. Setting a batch's shapes synchronises the device and records its
- * graphs again. */
+ * ray marcher being persistent), but for the tile order, whose 0 is an order
+ * of its own. Values above 64 (tile orders above 2) are refused. Setting a
+ * batch's shapes synchronises the device and records its graphs again. */
 typedef struct vmap_launch_config {
     int alloc_ctas_per_sm;
     int visibility_ctas_per_sm;
@@ -278,9 +278,9 @@ typedef struct vmap_launch_config {
     int normals_ctas_per_sm;
     int mesh_ctas_per_sm;
     /* order in which the ray marcher hands out each image's pixel tiles:
-     * 0 = default (alternating from both ends), 1 = top rows first, 2 =
-     * alternating from both ends. Tiles are independent, so only the time changes: the
-     * slowest tiles are best started first. */
+     * 0 = bottom rows first, 1 = top rows first, 2 = alternating from both
+     * ends, which maps and batches start with. Tiles are independent, so only
+     * the time changes: the slowest tiles are best started first. */
     int raycast_tile_order;
     /* ray-marcher tile: a warp marches a tile of 32 neighbouring rays,
      * raycast_tile_width pixels wide (4, 8 or 16; 0 = 8) and 32 / width

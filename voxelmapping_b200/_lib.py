@@ -61,7 +61,8 @@ class HostFrame(C.Structure):
 
 
 class LaunchConfig(C.Structure):
-    """vmap_launch_config: grid of every stage in CTAs per SM (0 = default)."""
+    """vmap_launch_config: grid of every stage in CTAs per SM (0 = default), the ray
+    marcher's tile and its order, a batch's schedule."""
     _fields_ = [("alloc_ctas_per_sm", C.c_int), ("visibility_ctas_per_sm", C.c_int), ("fuse_ctas_per_sm", C.c_int),
                 ("zrange_ctas_per_sm", C.c_int), ("raycast_ctas_per_sm", C.c_int), ("normals_ctas_per_sm", C.c_int),
                 ("mesh_ctas_per_sm", C.c_int), ("raycast_tile_order", C.c_int),

@@ -43,7 +43,7 @@ CANDIDATES = {
     "raycast_ctas_per_sm": [2, 3, 4, 0],
     "normals_ctas_per_sm": [2, 4, 8, 16],
     "mesh_ctas_per_sm": [4, 8, 16, 32],
-    "raycast_tile_order": [0, 1, 2],  # alternating ends (the default), top rows first, alternating ends
+    "raycast_tile_order": [0, 1, 2],  # bottom rows first, top rows first, alternating ends
     "raycast_tile_width": [8, 16, 4],  # 8x4, 16x2 or 4x8 rays per warp
     "raycast_threads_per_cta": [256, 128],
     "batch_schedule": [2, 1],  # one persistent launch per batch step, or one launch per stage

@@ -526,19 +526,28 @@ struct March {
     }
 };
 
+// The q-th of a map's nt tiles to be handed out, as a row-major index: order 0
+// bottom rows first, 1 top rows first, 2 alternating from both ends (what a map
+// starts with). The slow tiles are often those of the upper or the lower rows,
+// seen at grazing angles, and started last they prolong the launch: alternating
+// against bottom rows first 70 -> 64 us at 640x480, 131 -> 119 us for the 800x600
+// full march, 67 -> 64 us a view at 517x389, no difference at 320x240 and on
+// batches.
+__host__ __device__ constexpr int tile_at(int order, int q, int nt)
+{
+    return order == 0 ? nt - 1 - q : order == 1 ? q : (q & 1) ? nt - 1 - (q >> 1) : (q >> 1);
+}
+static_assert(tile_at(0, 0, 5) == 4 && tile_at(0, 4, 5) == 0 && tile_at(1, 0, 5) == 0 && tile_at(1, 4, 5) == 4 &&
+                  tile_at(2, 0, 5) == 0 && tile_at(2, 1, 5) == 4 && tile_at(2, 4, 5) == 2 && tile_at(2, 3, 4) == 2,
+              "three different orders, each of all tiles");
+
 // One warp marches tile q of the nt tiles of a map (q counts in the order the
 // tiles are handed out).
 template <int FMT, bool NC, bool WIDE>
 __device__ __forceinline__ void march_tile(const MapView& v, int q, int nt, int order, int tw, int lane)
 {
     typedef March<FMT, NC, WIDE> M;
-    // the map's q-th tile in the requested order (row-major tile index t): 1
-    // top rows first, 0 and 2 alternating from both ends. The slow tiles are
-    // often those of the upper or the lower rows, seen at grazing angles, and
-    // started last they prolong the launch: alternating against bottom rows
-    // first 70 -> 64 us at 640x480, 131 -> 119 us for the 800x600 full march,
-    // 67 -> 64 us a view at 517x389, no difference at 320x240 and on batches.
-    const int t = order == 1 ? q : (q & 1) ? nt - 1 - (q >> 1) : (q >> 1);
+    const int t = tile_at(order, q, nt);
     const int tx = (v.cam.W + tw - 1) / tw;
     const int x = (t % tx) * tw + (lane % tw), y = (t / tx) * (32 / tw) + (lane / tw);
     Ray r;

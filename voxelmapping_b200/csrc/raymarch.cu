@@ -26,7 +26,7 @@
 // Scheduling: the kernel is persistent. Each warp takes 8x4-pixel tiles from
 // one device-side queue shared by every map of the batch until it runs dry.
 // A map's tiles are handed out in a selectable order, alternating from both
-// ends of the image by default (march_tile).
+// ends of the image by default (tile_at).
 // (Refilling lanes from a larger group as their rays finish was measured
 // 2.8x slower: lanes at different depths scatter their loads and lookups.)
 #include "march.cuh"

@@ -26,7 +26,7 @@ struct Launcher {
     int alloc = 8, visibility = 2, fuse = 16, zrange = 4;
     int raycast = 0;  // persistent ray marcher: 0 = as many CTAs as fit on an SM
     int normals = 8, mesh = 8;
-    int tileOrder = 0;  // ray-marcher tile order (vmap_launch_config.raycast_tile_order)
+    int tileOrder = 2;  // ray-marcher tile order (vmap_launch_config.raycast_tile_order)
     int tileW = 8;       // ray-marcher tile width; the tile is 32 rays
     int rayThreads = 256;  // ray-marcher threads per CTA
     int batchSchedule = 1;  // vmap_launch_config.batch_schedule

@@ -111,7 +111,8 @@ class VoxelMapping:
         return {k: getattr(c, k) for k, _ in c._fields_}
 
     def set_launch_config(self, **kw):
-        """Sets some stages' grids (keys of get_launch_config; 0 = default)."""
+        """Sets some stages' grids (keys of get_launch_config; 0 = default, but for
+        raycast_tile_order: bottom rows first)."""
         cur = self.get_launch_config()
         cur.update(kw)
         L.check(self._lib.vmap_set_launch_config(self._need(), C.byref(L.LaunchConfig(**cur))),
