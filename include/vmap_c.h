@@ -267,8 +267,11 @@ vmap_status vmap_batch_stall_probe(vmap_batch* batch, const vmap_batch_frame* fr
  * 0 in a field selects the library default (alloc 8, visibility 2, fuse 16,
  * zrange 4, normals 8, mesh 8; raycast 0 = as many CTAs as fit on an SM, the
  * ray marcher being persistent), but for the tile order, whose 0 is an order
- * of its own. Values above 64 (tile orders above 2) are refused. Setting a
- * batch's shapes synchronises the device and records its graphs again. */
+ * of its own. Values above 64 (tile orders above 2) are refused. The ray
+ * marcher's and the mesh's grids end at what is resident (for the mesh 6 on the
+ * counting pass, 3.5 on the emitting one, in CTAs of 256 threads): larger values
+ * give the same launch. Setting a batch's shapes synchronises the device and
+ * records its graphs again. */
 typedef struct vmap_launch_config {
     int alloc_ctas_per_sm;
     int visibility_ctas_per_sm;

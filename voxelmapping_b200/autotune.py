@@ -42,7 +42,7 @@ CANDIDATES = {
     "zrange_ctas_per_sm": [1, 2, 4, 8],
     "raycast_ctas_per_sm": [2, 3, 4, 0],
     "normals_ctas_per_sm": [2, 4, 8, 16],
-    "mesh_ctas_per_sm": [4, 8, 16, 32],
+    "mesh_ctas_per_sm": [2, 3, 4, 8],  # 8: as many as fit (6 on the counting pass that is timed)
     "raycast_tile_order": [0, 1, 2],  # bottom rows first, top rows first, alternating ends
     "raycast_tile_width": [8, 16, 4],  # 8x4, 16x2 or 4x8 rays per warp
     "raycast_threads_per_cta": [256, 128],
