@@ -217,7 +217,30 @@ __global__ void __launch_bounds__(256) reset_kernel(DevMap m, bool whole)
     const size_t blocks = unknown ? (size_t)m.capacity : (size_t)allocated_blocks(m);
     const size_t words = blocks * (size_t)m.blockBytes / sizeof(uint4);
     uint4* w = reinterpret_cast<uint4*>(m.pool);
-    for (size_t i = t; i < words; i += nt) w[i] = make_uint4(0u, 0u, 0u, 0u);
+    // What L2 holds is written at a fixed stride, in even shares (8,192 blocks of
+    // 5,632 B: 28.3 us against 30.5 by chunks). More goes in chunks of 32 KB handed
+    // out in the order of their addresses: at a fixed stride the CTAs drift apart
+    // and DRAM is slower (2^18 blocks, 1.48 GB: 222 us against 267; 2^15 blocks 46
+    // against 49). Every chunk is followed by one take, so the queue's word wraps
+    // to zero with the last one.
+    if (words < (size_t)(120 << 20) / sizeof(uint4)) {
+        for (size_t i = t; i < words; i += nt) w[i] = make_uint4(0u, 0u, 0u, 0u);
+        return;
+    }
+    constexpr int kChunk = 8 * 256;
+    const unsigned chunks = (unsigned)((words + kChunk - 1) / kChunk);
+    __shared__ unsigned s_next;
+    for (unsigned c = blockIdx.x; c < chunks;) {
+        if (threadIdx.x == 0) s_next = gridDim.x + atomicInc(m.ctr + C_CLEARQ, chunks - 1);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            const size_t i = (size_t)c * kChunk + k * 256 + threadIdx.x;
+            if (i < words) w[i] = make_uint4(0u, 0u, 0u, 0u);
+        }
+        __syncthreads();
+        c = s_next;
+        __syncthreads();
+    }
 }
 
 // ------------------------------------------------------------------ launchers

@@ -42,6 +42,7 @@ enum {
     C_RAYQ = 8,    // raycast work queue of the single-map path
     C_LINKED = 9,  // blocks [0, C_LINKED) have their neighbour links set
     C_UNKNOWN = 10, // non-zero while a snapshot load runs: pool blocks beyond the allocated ones may hold data
+    C_CLEARQ = 11, // queue of the reset's pool chunks; zero outside the kernel
     C_COUNT = 16
 };
 
