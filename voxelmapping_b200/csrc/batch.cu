@@ -8,7 +8,7 @@
 // camera, frame pointers, FP32 poses, outputs) live in device memory and are
 // refreshed by one host-to-device copy per step from pinned staging, so the
 // whole step - copy plus six kernels - is recorded once as a CUDA graph and
-// replayed. Two staging buffers and two graphs alternate, so the host never
+// replayed. Two staging buffers and their graphs alternate, so the host never
 // rewrites descriptors a replay still has to copy.
 //
 // The reference has no counterpart: VoxelMapping drives one map per call.
@@ -31,7 +31,17 @@ cudaError_t next_epoch(vmap_map* m, cudaStream_t s, unsigned* epoch);
 struct StepForms {
     bool near;  // allocation: every fused view is near
     bool wide;  // ray marcher: some rendered view is wide
-    bool operator!=(const StepForms& o) const { return near != o.near || wide != o.wide; }
+    int index() const { return (near ? 1 : 0) + (wide ? 2 : 0); }
+};
+constexpr int kStepForms = 4;
+
+// A recorded step: a graph for each staging buffer and each combination of
+// kernel forms, recorded when a step first needs it. (One graph a buffer,
+// recorded anew whenever the forms change, took 155 us of host time each: a step
+// of 16 maps at 320x240 alone 722 us against 549.)
+struct StepGraph {
+    cudaGraphExec_t exec;
+    cudaStream_t stream;  // it was recorded for
 };
 
 struct vmap_batch {
@@ -46,9 +56,7 @@ struct vmap_batch {
     StepSched* dSched;       // scheduler of the persistent step
     cudaEvent_t copied[2];   // the copy out of staging b has executed
     bool eventUsed[2];
-    cudaGraphExec_t exec[2];
-    cudaStream_t graphStream[2];  // stream each graph was recorded for
-    StepForms graphForms[2];      // kernel forms it was recorded with
+    StepGraph graphs[2][kStepForms];
     int next;                // buffer of the next step
 };
 
@@ -66,10 +74,20 @@ vmap_status fail(cudaError_t e, const char* what)
         if (e_ != cudaSuccess) return fail(e_, #expr);      \
     } while (0)
 
+// The next step of every buffer and form records its graph again.
+void drop_graphs(vmap_batch* b)
+{
+    for (StepGraph(&of)[kStepForms] : b->graphs)
+        for (StepGraph& g : of) {
+            if (g.exec) cudaGraphExecDestroy(g.exec);
+            g = StepGraph{};
+        }
+}
+
 void release(vmap_batch* b)
 {
+    drop_graphs(b);
     for (int i = 0; i < 2; ++i) {
-        if (b->exec[i]) cudaGraphExecDestroy(b->exec[i]);
         if (b->copied[i]) cudaEventDestroy(b->copied[i]);
         cudaFree(b->dViews[i]);
         if (b->hViews[i]) cudaFreeHost(b->hViews[i]);
@@ -187,11 +205,7 @@ vmap_status vmap_batch_set_map(vmap_batch* b, int slot, vmap_map* map)
         // grids were sized for the original maps: from now on launch full
         // grids, and record the graphs again once the steps in flight are done
         VMAP_BCK(cudaDeviceSynchronize());
-        for (int i = 0; i < 2; ++i)
-            if (b->exec[i]) {
-                cudaGraphExecDestroy(b->exec[i]);
-                b->exec[i] = nullptr;
-            }
+        drop_graphs(b);
         b->totalAllocTiles = b->totalNormalTiles = kFullGrid;
     }
     b->maps[slot] = map;
@@ -210,11 +224,7 @@ vmap_status vmap_batch_set_launch_config(vmap_batch* b, const vmap_launch_config
     if (!b || !cfg || !launch_config_ok(cfg)) return VMAP_ERR_INVALID_ARG;
     // the recorded graphs hold the old grids: record again once the steps in flight are done
     VMAP_BCK(cudaDeviceSynchronize());
-    for (int i = 0; i < 2; ++i)
-        if (b->exec[i]) {
-            cudaGraphExecDestroy(b->exec[i]);
-            b->exec[i] = nullptr;
-        }
+    drop_graphs(b);
     launch_config_to(cfg, b->launcher);
     return VMAP_OK;
 }
@@ -313,11 +323,12 @@ vmap_status vmap_batch_step(vmap_batch* b, const vmap_batch_frame* frames, void*
         VMAP_BCK(cudaEventRecord(b->copied[buf], s));
         VMAP_BCK(enqueue_stages(b, buf, forms, s));
     } else {
-        if (b->exec[buf] && (b->graphStream[buf] != s || b->graphForms[buf] != forms)) {
-            cudaGraphExecDestroy(b->exec[buf]);
-            b->exec[buf] = nullptr;
+        StepGraph& r = b->graphs[buf][forms.index()];
+        if (r.exec && r.stream != s) {
+            cudaGraphExecDestroy(r.exec);
+            r.exec = nullptr;
         }
-        if (!b->exec[buf]) {
+        if (!r.exec) {
             cudaGraph_t g = nullptr;
             VMAP_BCK(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
             cudaError_t e = cudaMemcpyAsync(b->dViews[buf], b->hViews[buf], bytes, cudaMemcpyHostToDevice, s);
@@ -326,13 +337,15 @@ vmap_status vmap_batch_step(vmap_batch* b, const vmap_batch_frame* frames, void*
             if (e == cudaSuccess) e = enqueue_stages(b, buf, forms, s);
             cudaError_t e2 = cudaStreamEndCapture(s, &g);
             if (e == cudaSuccess) e = e2;
-            if (e == cudaSuccess) e = cudaGraphInstantiate(&b->exec[buf], g, 0);
+            if (e == cudaSuccess) e = cudaGraphInstantiate(&r.exec, g, 0);
             if (g) cudaGraphDestroy(g);
-            if (e != cudaSuccess) return fail(e, "vmap_batch_step capture");
-            b->graphStream[buf] = s;
-            b->graphForms[buf] = forms;
+            if (e != cudaSuccess) {
+                r.exec = nullptr;
+                return fail(e, "vmap_batch_step capture");
+            }
+            r.stream = s;
         }
-        VMAP_BCK(cudaGraphLaunch(b->exec[buf], s));
+        VMAP_BCK(cudaGraphLaunch(r.exec, s));
     }
     b->eventUsed[buf] = true;
     b->next = buf ^ 1;
