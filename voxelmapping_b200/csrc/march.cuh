@@ -68,6 +68,13 @@ struct March {
         return valid ? F::tsdf(w) : 1.f;
     }
 
+    static __device__ __forceinline__ float voxel(const DevMap& m, int slot, int ix, int iy, int iz, bool& valid)
+    {
+        if (slot >= 0) return value(ld_map<NC>(Layout<FMT>::words(m, slot) + at(ix, iy, iz)), valid);
+        valid = false;
+        return 1.f;
+    }
+
     // Block coordinates of a floor code. Narrow codes themselves agree with
     // the coordinates in the bits that the grid's cells and tags use.
     static __device__ __forceinline__ int block(int i)
@@ -313,9 +320,7 @@ struct March {
         r.y = y;
         r.sdf = 1.f;
         r.valid = false;
-        // a region of its own: every code differs from it above the low 3 bits
-        // (a wide one only from 2^31 voxels down does not, where no block can be)
-        r.cx = r.cy = r.cz = INT_MIN;
+        r.cx = r.cy = r.cz = INT_MIN;  // a region of its own: no sample's codes have this top bit
         r.cmask = 7;
         r.cblk = -1;
         return true;
@@ -489,18 +494,23 @@ struct March {
             const int ix = fl(r.res.x), iy = fl(r.res.y), iz = fl(r.res.z);
             int slot = r.cblk;
             if (moved(r, ix, iy, iz) & ~7) slot = find(v.m, ix, iy, iz);
-            bool valid = false;  // corner 0 is unobserved where its block is not allocated: a miss
+            bool valid = false;
             const Corners c = corners(r.res, ix, iy, iz);
             const int cross = c.cross();
             float e[8];
             if (slot >= 0) {
                 const Word w0 = ld_map<NC>(Layout<FMT>::words(v.m, slot) + at(ix, iy, iz));
                 valid = corners8(v.m, slot, far_slot(v.m, slot, cross), cross, c, w0, e);
-            } else {
+            } else {  // corner 0's block is not allocated: the read is invalid, its value still counts
 #pragma unroll
-                for (int k = 0; k < 8; ++k) e[k] = 1.f;
+                for (int k = 0; k < 8; ++k) {
+                    const int vx = (k & 1) ? c.x1 : c.x0, vy = (k & 2) ? c.y1 : c.y0, vz = (k & 4) ? c.z1 : c.z0;
+                    bool ok;
+                    e[k] = k & cross ? voxel(v.m, find(v.m, vx, vy, vz), vx, vy, vz, ok) : 1.f;
+                }
             }
-            r.res = fma3(__fmul_rn(lerp8(e, c.ax, c.ay, c.az), o.rts), r.dir, r.res);
+            const float s = lerp8(e, c.ax, c.ay, c.az);
+            r.res = fma3(__fmul_rn(s, o.rts), r.dir, r.res);
             found = valid;
         }
         float4 out;
