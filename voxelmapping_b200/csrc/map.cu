@@ -164,8 +164,10 @@ void make_view(const vmap_map* m, const double pose[16], MapView& v)
         v.out.wide = !m->dm.grid || !(reach < narrow_limit(m->dm.g));
         // a jump rounds a position by half a unit in the last place, 2^-24 of
         // it; the 48 block faces of the widest cube take at most 96 jumps (one
-        // that stops short of a face is followed by a step of one voxel)
-        v.out.slack = (float)(0.05 + reach * 0x1p-17);
+        // that stops short of a face is followed by a step of one voxel). The
+        // limit's own rounding, on up to 128 voxels, is below 2^-14 voxels and 2
+        // half units of the position.
+        v.out.slack = (float)(0x1p-8 + reach * 0x1p-17);
     }
     v.out.mode = m->cfg.raycast_mode;
 }

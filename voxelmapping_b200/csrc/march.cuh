@@ -320,7 +320,9 @@ struct March {
         r.y = y;
         r.sdf = 1.f;
         r.valid = false;
-        r.cx = r.cy = r.cz = INT_MIN;  // a region of its own: no sample's codes have this top bit
+        // a region of its own: every code differs from it above the low 3 bits
+        // (a wide one only from 2^31 voxels down does not, where no block can be)
+        r.cx = r.cy = r.cz = INT_MIN;
         r.cmask = 7;
         r.cblk = -1;
         return true;
@@ -501,7 +503,11 @@ struct March {
             if (slot >= 0) {
                 const Word w0 = ld_map<NC>(Layout<FMT>::words(v.m, slot) + at(ix, iy, iz));
                 valid = corners8(v.m, slot, far_slot(v.m, slot, cross), cross, c, w0, e);
-            } else {  // corner 0's block is not allocated: the read is invalid, its value still counts
+            } else {
+                // corner 0's block is not allocated: the read is invalid and the
+                // pixel a miss, whatever the corners hold. (As a branch of its
+                // own, without these lookups, the kernel was compiled to run
+                // 0.5-1.4 % slower on the cases of several sizes, 4 % in one form.)
 #pragma unroll
                 for (int k = 0; k < 8; ++k) {
                     const int vx = (k & 1) ? c.x1 : c.x0, vy = (k & 2) ? c.y1 : c.y0, vz = (k & 4) ? c.z1 : c.z0;

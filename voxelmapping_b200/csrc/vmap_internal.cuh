@@ -189,7 +189,7 @@ __device__ __forceinline__ int local_idx(int vx, int vy, int vz)
 // few buckets may have none; its lookups go to the hash table.
 constexpr unsigned kGridValid = 1u << 30, kGridShared = 1u << 31;  // in an entry's high word
 
-// bytes of a grid of 2^k cells: entries, brick words, region words
+// 8-byte words of a grid of 2^k cells: entries, brick words, region words
 __host__ __device__ constexpr size_t grid_words(int k)
 {
     return ((size_t)1 << k) + ((size_t)1 << (k - 6)) + (k > 15 ? (size_t)1 << (k - 12) : 8);
