@@ -65,6 +65,7 @@ namespace {
 vmap_status fail(cudaError_t e, const char* what)
 {
     set_last_error(std::string(what) + ": " + cudaGetErrorString(e));
+    cudaGetLastError();  // reported here: the next launch's check is not to find it again
     return e == cudaErrorMemoryAllocation ? VMAP_ERR_OUT_OF_MEMORY : VMAP_ERR_CUDA;
 }
 

@@ -75,6 +75,7 @@ extern "C" vmap_status vmap_export_blocks_static(vmap_map* map, uint32_t first, 
     cudaError_t e = stage_address(&base);
     if (e != cudaSuccess) {
         set_last_error(std::string("vmap_export_blocks_static: ") + cudaGetErrorString(e));
+        cudaGetLastError();  // reported here: the next launch's check is not to find it again
         return VMAP_ERR_CUDA;
     }
     int* d_coords = reinterpret_cast<int*>(base);
@@ -96,6 +97,7 @@ extern "C" vmap_status vmap_export_blocks_static(vmap_map* map, uint32_t first, 
     if (e == cudaSuccess) e = cudaStreamSynchronize(cs);
     if (e != cudaSuccess) {
         set_last_error(std::string("vmap_export_blocks_static: ") + cudaGetErrorString(e));
+        cudaGetLastError();  // reported here: the next launch's check is not to find it again
         return VMAP_ERR_CUDA;
     }
     return VMAP_OK;

@@ -63,6 +63,7 @@ thread_local std::string g_last_error;
 vmap_status cuda_fail(cudaError_t e, const char* what)
 {
     g_last_error = std::string(what) + ": " + cudaGetErrorString(e);
+    cudaGetLastError();  // reported here: the next launch's check is not to find it again
     return e == cudaErrorMemoryAllocation ? VMAP_ERR_OUT_OF_MEMORY : VMAP_ERR_CUDA;
 }
 

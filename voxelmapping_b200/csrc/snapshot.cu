@@ -37,6 +37,7 @@ vmap_status fail(vmap_status st, const std::string& msg)
 vmap_status cuda_fail(cudaError_t e, const char* what)
 {
     set_last_error(std::string(what) + ": " + cudaGetErrorString(e));
+    cudaGetLastError();  // reported here: the next launch's check is not to find it again
     return e == cudaErrorMemoryAllocation ? VMAP_ERR_OUT_OF_MEMORY : VMAP_ERR_CUDA;
 }
 

@@ -23,7 +23,9 @@ void check(vmap_status s, const char* what)
 
 void check_cuda(cudaError_t e, const char* what)
 {
-    if (e != cudaSuccess) throw Error(VMAP_ERR_CUDA, std::string(what) + ": " + cudaGetErrorString(e));
+    if (e == cudaSuccess) return;
+    cudaGetLastError();  // reported here: the next launch's check is not to find it again
+    throw Error(VMAP_ERR_CUDA, std::string(what) + ": " + cudaGetErrorString(e));
 }
 
 void to_pose(const Mat4f& m, double* p)
